@@ -3,15 +3,18 @@
 // The reference's permute_rmw issues one global atomic read-modify-write per
 // source element (accelerate-llvm-ptx/src/Data/Array/Accelerate/LLVM/PTX/
 // CodeGen/Permute.hs:117-213), so a skewed (Zipf) histogram serialises on the
-// few hot bins in L2.  Two kernels here:
+// few hot bins in L2.  Kernels here:
+//   * permute_count32 / permute_count16 -- integer + of a constant (histograms):
+//     private counters in shared memory, 32 bits per bin while they fit, else
+//     16 bits; the constant multiplies the counts once, at the end;
+//   * permute_private -- every other update of a target that fits in shared
+//     memory: a private copy of the target per CTA, folded into global memory
+//     at the end;
+//   * permute_cluster -- for 32-bit integer targets beyond that, up to 8 x 48K
+//     bins: the target is privatised in the DISTRIBUTED shared memory of a
+//     thread-block cluster (each CTA of the cluster holds 1/CL of the bins);
 //   * permute_global -- red.global / atom.global RMW per element (any type,
-//     any primitive; CAS loops for the primitives without a native atomic);
-//   * permute_cluster -- for 32-bit integer targets up to 8 x 50K bins: the
-//     target array is privatised in the DISTRIBUTED shared memory of a
-//     thread-block cluster (each CTA of the cluster holds 1/CL of the bins,
-//     filled with the identity), every element does a shared-memory atomic
-//     on the CTA that owns its bin, and at the end each CTA folds its bins
-//     into global memory with one atomic per touched bin.
+//     any primitive; CAS loops for the primitives without a native atomic).
 // Each update is out[j] = f x out[j] with the new value first, the order of
 // the reference's combine (Native/CodeGen/Permute.hs:112-116).  Integer
 // results do not depend on the update order; Float32/Float64 + does.
@@ -33,6 +36,7 @@ struct PermArgs {
   uint64_t cval;
   int has_src;
   int idx64;
+  int vec;  // idx and src are 16-byte aligned
   uint32_t *err;
 };
 
@@ -79,6 +83,7 @@ __device__ __forceinline__ void atomic_combine(T *p, T x) {
       do {
         assumed = old;
         float nv = Prim<OP, float>::ap(x, __uint_as_float(assumed));
+        if (__float_as_uint(nv) == assumed) break;  // min / max: already there
         old = atomicCAS(q, assumed, __float_as_uint(nv));
       } while (old != assumed);
     }
@@ -90,6 +95,7 @@ __device__ __forceinline__ void atomic_combine(T *p, T x) {
       do {
         assumed = old;
         double nv = Prim<OP, double>::ap(x, __longlong_as_double((long long)assumed));
+        if ((unsigned long long)__double_as_longlong(nv) == assumed) break;
         old = atomicCAS(q, assumed, (unsigned long long)__double_as_longlong(nv));
       } while (old != assumed);
     }
@@ -100,19 +106,389 @@ __device__ __forceinline__ int64_t perm_idx(const PermArgs &a, int64_t i) {
   return a.idx64 ? static_cast<const int64_t *>(a.idx)[i] : (int64_t) static_cast<const int32_t *>(a.idx)[i];
 }
 
+// Four source elements of a round, in registers: their target indices as
+// Int32 (negative: Nothing; a 64-bit index at or past m, which the shared
+// memory kernels keep below 2^31, becomes m) and their values.  Unit v is the
+// four consecutive elements 4v.. read with 16-byte loads, or four single
+// elements.  FIXED: the array forms are known at compile time (IDX64, no
+// source); otherwise the flags of PermArgs decide, the same for every thread.
+template <class T, bool FIXED = false, bool IDX64 = false> struct PermUnit {
+  int32_t j[4];
+  T x[4];
+  __device__ __forceinline__ static bool idx64(const PermArgs &a) { return FIXED ? IDX64 : a.idx64 != 0; }
+  __device__ __forceinline__ static bool src(const PermArgs &a) { return FIXED ? false : a.has_src != 0; }
+  __device__ __forceinline__ void clear(T c) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { j[k] = -1; x[k] = c; }
+  }
+  __device__ __forceinline__ static int32_t narrow(int64_t j, int64_t m) {
+    return j < 0 ? -1 : (j >= m ? (int32_t)m : (int32_t)j);
+  }
+  // ip, sp: the unit's first index and value
+  __device__ __forceinline__ void load_vec(const PermArgs &a, const char *ip, const char *sp, T c) {
+    if (idx64(a)) {
+      const uint4 *p = reinterpret_cast<const uint4 *>(ip);
+      const uint4 q0 = ld_stream16(p), q1 = ld_stream16(p + 1);
+      int64_t w[4];
+      memcpy(w, &q0, 16);
+      memcpy(w + 2, &q1, 16);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) j[k] = narrow(w[k], a.m);
+    } else {
+      const uint4 q = ld_stream16(ip);
+      memcpy(j, &q, 16);
+    }
+    if (src(a)) {
+      constexpr int Q = sizeof(T) / 4;
+      uint4 q[Q];
+#pragma unroll
+      for (int k = 0; k < Q; ++k) q[k] = ld_stream16(reinterpret_cast<const uint4 *>(sp) + k);
+      memcpy(x, q, sizeof(x));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) x[k] = c;
+    }
+  }
+  __device__ __forceinline__ void load_el(const PermArgs &a, int k, int64_t e) {
+    if (idx64(a)) j[k] = narrow(ld_stream(static_cast<const int64_t *>(a.idx) + e), a.m);
+    else j[k] = ld_stream(static_cast<const int32_t *>(a.idx) + e);
+    if (src(a)) x[k] = ld_stream(static_cast<const T *>(a.src) + e);
+  }
+};
+
+// Stream the source once over the whole grid: every thread gets U units per
+// round and calls batch(units) convergently (the lanes of a warp run the same
+// rounds; what a round lacks holds index -1).  The next round's loads are in
+// flight while a round's updates run: an update's returned value is waited
+// for, so without that the loads would start only after the last return
+// (permute_count16, 2^28 uniform / Zipf indices: 0.205 / 0.220 ms with four
+// units and no prefetch, 0.168 / 0.178 with two prefetched units).
+// The source is read with 16-byte loads where idx and src are 16-byte aligned
+// (a.vec), else element by element, each load coalesced over the warp.
+template <class Unit, int U, class T, class F>
+__device__ __forceinline__ void perm_stream(const PermArgs &a, T c, F &&batch) {
+  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t nth = (int64_t)gridDim.x * blockDim.x;
+  const int64_t nunits = a.n / 4;
+  const int64_t per = a.vec ? U * nth : 4 * U * nth;   // units, or elements, per round
+  const int64_t whole = a.vec ? nunits / per : 0;      // rounds in which every unit exists
+  const int64_t rounds = a.vec ? (nunits + per - 1) / per + ((a.n & 3) ? 1 : 0) : (a.n + per - 1) / per;
+  const int64_t ib = Unit::idx64(a) ? 32 : 16, sb = Unit::src(a) ? 4 * (int64_t)sizeof(T) : 0;  // bytes of a unit
+  const char *ip = static_cast<const char *>(a.idx) + tid * ib;
+  const char *sp = static_cast<const char *>(a.src) + tid * sb;
+  auto load_whole = [&](Unit (&q)[U]) {  // the next round, every unit of it
+#pragma unroll
+    for (int u = 0; u < U; ++u) q[u].load_vec(a, ip + u * nth * ib, sp + u * nth * sb, c);
+    ip += per * ib;
+    sp += per * sb;
+  };
+  Unit next[U];
+  if (whole > 0) load_whole(next);
+  for (int64_t r = 0; r < whole; ++r) {
+    Unit q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) q[u] = next[u];
+    if (r + 1 < whole) load_whole(next);
+    batch(q);
+  }
+  for (int64_t r = whole; r < rounds; ++r) {
+    Unit q[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) q[u].clear(c);
+    if (!a.vec) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int64_t e = r * per + (u * 4 + k) * nth + tid;
+          if (e < a.n) q[u].load_el(a, k, e);
+        }
+    } else if (r * per < nunits) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if ((r * U + u) * nth + tid < nunits) q[u].load_vec(a, ip + u * nth * ib, sp + u * nth * sb, c);
+    } else if (4 * nunits + tid < a.n) {
+      q[0].load_el(a, 0, 4 * nunits + tid);  // the last n % 4 elements
+    }
+    batch(q);
+  }
+}
+
 template <int OP, class T>
 __global__ void __launch_bounds__(256) permute_global(PermArgs a) {
   const T *src = static_cast<const T *>(a.src);
   T *out = static_cast<T *>(a.out);
   const T c = from_bits<T>(a.cval);
+  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t nth = (int64_t)gridDim.x * blockDim.x;
   bool bad = false;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t j = perm_idx(a, i);
-    if (j < 0) continue;  // Nothing: the element is dropped
-    if (j >= a.m) { bad = true; continue; }
-    atomic_combine<OP, T>(out + j, a.has_src ? src[i] : c);
+  auto one = [&](int64_t j, T x) {
+    if (j < 0) return;  // Nothing: the element is dropped
+    if (j >= a.m) { bad = true; return; }
+    atomic_combine<OP, T>(out + j, x);
+  };
+  int64_t e0 = 0;
+  if (a.vec) {
+    // 16-byte loads of four indices and four values.
+    for (int64_t v = tid; v < a.n / 4; v += nth) {
+      int64_t j[4];
+      T x[4];
+      if (a.idx64) {
+        const uint4 q0 = ld_stream16(static_cast<const uint4 *>(a.idx) + 2 * v);
+        const uint4 q1 = ld_stream16(static_cast<const uint4 *>(a.idx) + 2 * v + 1);
+        memcpy(j, &q0, 16);
+        memcpy(j + 2, &q1, 16);
+      } else {
+        const uint4 q = ld_stream16(static_cast<const uint4 *>(a.idx) + v);
+        int32_t w[4];
+        memcpy(w, &q, 16);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) j[k] = w[k];
+      }
+      if (a.has_src) {
+        constexpr int Q = sizeof(T) / 4;
+        uint4 q[Q];
+#pragma unroll
+        for (int k = 0; k < Q; ++k) q[k] = ld_stream16(static_cast<const uint4 *>(a.src) + Q * v + k);
+        memcpy(x, q, sizeof(x));
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) one(j[k], a.has_src ? x[k] : c);
+    }
+    e0 = a.n / 4 * 4;
   }
+  for (int64_t i = e0 + tid; i < a.n; i += nth) one(perm_idx(a, i), a.has_src ? src[i] : c);
   if (bad) raise_error(a.err, DEV_ERR_INDEX);
+}
+
+// ----------------------------------------------------------------- shared-memory counters
+// Histograms (integer + of a constant c): bin j counts its updates and the
+// target gets c * count once, which is the same wrapping sum.  One CTA of
+// 1024 threads per SM holds all the bins.  Measured on a GB300, 2^28 Int32
+// indices (floor 158 us): an increment by a constant 1 whose result is not
+// used costs no more than reading the counter would (0.158-0.163 ms
+// against 0.153-0.161 for a plain load), same-address lanes included, so the
+// kernels are bound by reading the indices and by issue, and what an update
+// does besides its increment is what counts.
+constexpr int PERM_THREADS = 1024;
+constexpr int PERM_U = 2;  // units of four elements per thread and round
+
+// 32 bits per bin.  A counter may wrap mod 2^32 only beyond 2^32 updates per
+// CTA, where the 32-bit targets wrap as well and a 64-bit target's source
+// could not be in memory.
+template <class T, bool I64>
+__global__ void __launch_bounds__(PERM_THREADS, 1) permute_count32(PermArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint32_t *bins = reinterpret_cast<uint32_t *>(smem_raw);
+  const uint32_t m = (uint32_t)a.m;
+  for (uint32_t b = threadIdx.x; b < m; b += PERM_THREADS) bins[b] = 0u;
+  __syncthreads();
+  int32_t top = -1;
+  using Unit = PermUnit<uint32_t, true, I64>;
+  perm_stream<Unit, PERM_U>(a, 0u, [&](const Unit (&q)[PERM_U]) {
+#pragma unroll
+    for (int u = 0; u < PERM_U; ++u)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int32_t j = q[u].j[k];
+        top = j > top ? j : top;
+        if ((uint32_t)j < m) atomicAdd(bins + j, 1u);
+      }
+  });
+  if (top >= (int32_t)m) raise_error(a.err, DEV_ERR_INDEX);
+  __syncthreads();
+  T *out = static_cast<T *>(a.out);
+  const T c = from_bits<T>(a.cval);
+  for (uint32_t b = threadIdx.x; b < m; b += PERM_THREADS) {
+    const uint32_t n = bins[b];
+    if (n) atomic_combine<ACC_ADD, T>(out + b, Prim<ACC_MUL, T>::ap((T)n, c));
+  }
+}
+
+// 16 bits per bin, two to a word: bin w in the low half of word w and bin
+// w + half in its high half, half = ceil(m / 2), so that neighbouring bins,
+// which skewed (Zipf-like) indices make hot together, sit in different banks.
+// No counter ever wraps: a counter at or above 0x8000 (its guard bit) is
+// moved to the target.  Every update returns the word it found; a thread
+// tests the OR of its batch of 8 once, and if a guard bit was set it takes
+// each still-guarded word of the batch with an exchange and adds both
+// counters to the target.  Until the first such exchange after a counter
+// reaches 0x8000, a thread can add at most its current batch to it (any
+// update after the crossing sees the guard), so the counter stays below
+// 0x8000 + 1024 * 8 < 2^16.
+// 2^28 Zipf(1.1) indices to 2^16 bins: a wrap test and repair per update took
+// 0.257 ms, this 0.202 ms (uniform indices 0.176); a barrier and a sweep of the words every 32 updates
+// 0.29 ms; 57,344 32-bit counters with only the remaining bins packed into
+// high halves 0.34 ms (two divergent updates per index).
+template <class T, bool I64>
+__global__ void __launch_bounds__(PERM_THREADS, 1) permute_count16(PermArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  uint32_t *words = reinterpret_cast<uint32_t *>(smem_raw);
+  constexpr uint32_t GUARD = 0x80008000u;
+  const uint32_t m = (uint32_t)a.m, half = (m + 1) / 2;
+  for (uint32_t b = threadIdx.x; b < half; b += PERM_THREADS) words[b] = 0u;
+  __syncthreads();
+  T *out = static_cast<T *>(a.out);
+  const T c = from_bits<T>(a.cval);
+  auto flush = [&](uint32_t w, uint32_t v) {
+    if (v & 0xffffu) atomic_combine<ACC_ADD, T>(out + w, Prim<ACC_MUL, T>::ap((T)(v & 0xffffu), c));
+    if (v >> 16) atomic_combine<ACC_ADD, T>(out + w + half, Prim<ACC_MUL, T>::ap((T)(v >> 16), c));
+  };
+  int32_t top = -1;
+  using Unit = PermUnit<uint32_t, true, I64>;
+  perm_stream<Unit, PERM_U>(a, 0u, [&](const Unit (&q)[PERM_U]) {
+    uint32_t seen = 0u;
+#pragma unroll
+    for (int u = 0; u < PERM_U; ++u)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int32_t j = q[u].j[k];
+        top = j > top ? j : top;
+        const bool low = (uint32_t)j < half;
+        const uint32_t w = low ? (uint32_t)j : (uint32_t)j - half;
+        if ((uint32_t)j < m) seen |= atomicAdd(words + w, low ? 1u : 0x10000u);
+      }
+    if (seen & GUARD) {
+#pragma unroll
+      for (int u = 0; u < PERM_U; ++u)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int32_t j = q[u].j[k];
+          if ((uint32_t)j >= m) continue;
+          const uint32_t w = (uint32_t)j < half ? (uint32_t)j : (uint32_t)j - half;
+          if (*reinterpret_cast<volatile uint32_t *>(words + w) & GUARD) flush(w, atomicExch(words + w, 0u));
+        }
+    }
+  });
+  if (top >= (int32_t)m) raise_error(a.err, DEV_ERR_INDEX);
+  __syncthreads();
+  for (uint32_t b = threadIdx.x; b < half; b += PERM_THREADS) flush(b, words[b]);
+}
+
+// ----------------------------------------------------------------- private target
+// A private copy of the target in shared memory (identity-filled), one CTA of
+// 1024 threads per SM; at the end each CTA folds its touched bins into the
+// target.  L2 takes about 0.15 updates/ns whatever the target and one update
+// per 1.5 ns on a single address; shared memory takes five times that.
+// 2 * 10^7 Float32 values by 5 * 10^4 uniform keys: 0.166 -> 0.050 ms; 6.4 *
+// 10^6 Int64 values by 25,000: 0.057 -> 0.029 ms.  With four updates per bin
+// (the least that comes here) both ways take the time of a call.
+//
+// 64-bit integer bins are kept as two 32-bit words (all low words first), each
+// updated by a native 32-bit atomic: + adds the low halves, sees its carry in
+// the returned word and adds it with the high halves (0.06 ms for 2 * 10^7
+// values against 0.06-0.11 with the 64-bit compare-and-swap that atomicAdd is
+// there, and 0.06 against 0.6 ms under Zipf keys); and / or / xor are
+// bitwise.  64-bit min / max and the floats are compare-and-swap loops.
+template <int OP, class T> constexpr bool split64() {
+  return std::is_same<T, int64_t>::value && (OP == ACC_ADD || OP == ACC_AND || OP == ACC_OR || OP == ACC_XOR);
+}
+// Float + is a compare-and-swap loop that serialises lanes and warps on a hot
+// bin: lanes of a warp with the same key are added up first where keys repeat.
+template <int OP, class T> constexpr bool perm_aggregates() { return OP == ACC_ADD && is_fp<T>(); }
+
+template <int OP, class T>
+__device__ __forceinline__ void private_update(unsigned char *bins, uint32_t m, uint32_t j, T x) {
+  if constexpr (split64<OP, T>()) {
+    uint32_t *lo = reinterpret_cast<uint32_t *>(bins) + j, *hi = lo + m;
+    const uint32_t xl = (uint32_t)(uint64_t)x, xh = (uint32_t)((uint64_t)x >> 32);
+    if constexpr (OP == ACC_ADD) {
+      const uint32_t old = atomicAdd(lo, xl);
+      atomicAdd(hi, xh + (old + xl < xl ? 1u : 0u));
+    } else if constexpr (OP == ACC_AND) { atomicAnd(lo, xl); atomicAnd(hi, xh); }
+    else if constexpr (OP == ACC_OR) { atomicOr(lo, xl); atomicOr(hi, xh); }
+    else { atomicXor(lo, xl); atomicXor(hi, xh); }
+  } else {
+    atomic_combine<OP, T>(reinterpret_cast<T *>(bins) + j, x);
+  }
+}
+template <int OP, class T>
+__device__ __forceinline__ T private_bin(const unsigned char *bins, uint32_t m, uint32_t j) {
+  if constexpr (split64<OP, T>()) {
+    const uint32_t *lo = reinterpret_cast<const uint32_t *>(bins) + j;
+    return (T)((uint64_t)lo[0] | ((uint64_t)lo[m] << 32));
+  } else {
+    return reinterpret_cast<const T *>(bins)[j];
+  }
+}
+
+template <int OP, class T>
+__global__ void __launch_bounds__(PERM_THREADS, 1) permute_private(PermArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const uint32_t m = (uint32_t)a.m;
+  const T idT = Prim<OP, T>::id();
+  if constexpr (split64<OP, T>()) {
+    // both halves of the identity (0 or all ones) are the same word
+    for (uint32_t b = threadIdx.x; b < 2 * m; b += PERM_THREADS)
+      reinterpret_cast<uint32_t *>(smem_raw)[b] = (uint32_t)(uint64_t)idT;
+  } else {
+    for (uint32_t b = threadIdx.x; b < m; b += PERM_THREADS) reinterpret_cast<T *>(smem_raw)[b] = idT;
+  }
+  __syncthreads();
+  const T c = from_bits<T>(a.cval);
+  const int lane = threadIdx.x & 31;
+  int32_t top = -1;
+  uint32_t round = 0;
+  bool repeats = false;
+  using Unit = PermUnit<T>;
+  perm_stream<Unit, PERM_U>(a, c, [&](const Unit (&q)[PERM_U]) {
+    if constexpr (perm_aggregates<OP, T>()) {
+      // Every 8th round the warp looks at two of its updates: a key that three
+      // lanes share turns the aggregation on (uniform keys over 256 bins do
+      // that in 15 % of the looks, Zipf(1.1) keys in 85 %).  2 * 10^7 Float32
+      // values, uniform / Zipf keys over 5 * 10^4 bins: always 0.172 / 0.165
+      // ms, never 0.045 / 0.350 ms.
+      if ((round++ & 7u) == 0u) {
+        const unsigned g0 = __match_any_sync(0xffffffffu, q[0].j[0]), g1 = __match_any_sync(0xffffffffu, q[PERM_U - 1].j[3]);
+        const bool three = (q[0].j[0] >= 0 && __popc(g0) > 2) || (q[PERM_U - 1].j[3] >= 0 && __popc(g1) > 2);
+        repeats = __any_sync(0xffffffffu, three);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < PERM_U; ++u)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int32_t j = q[u].j[k];
+        top = j > top ? j : top;
+        T x = q[u].x[k];
+        bool mine = (uint32_t)j < m;
+        if constexpr (perm_aggregates<OP, T>()) {
+          if (repeats) {  // warp-uniform
+            const unsigned grp = __match_any_sync(0xffffffffu, j);
+            unsigned rest = grp & (grp - 1u);  // the peers after the first lane
+            const T own = x;
+            while (__any_sync(0xffffffffu, rest != 0u)) {
+              const T o = shfl_idx(own, rest ? __ffs(rest) - 1 : lane);
+              if (rest) x = Prim<OP, T>::ap(x, o);
+              rest &= rest - 1u;
+            }
+            mine = mine && (__ffs(grp) - 1) == lane;
+          }
+        }
+        if (mine) private_update<OP, T>(smem_raw, m, (uint32_t)j, x);
+      }
+  });
+  if (top >= (int32_t)m) raise_error(a.err, DEV_ERR_INDEX);
+  __syncthreads();
+
+  // Fold this CTA's bins into the target; untouched bins hold the identity.
+  T *out = static_cast<T *>(a.out);
+  uint32_t b0 = 0;
+  if constexpr (OP == ACC_ADD && std::is_same<T, float>::value) {
+    // four bins per reduction (an untouched bin's -0.0 changes nothing)
+    if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+      b0 = m & ~3u;
+      for (uint32_t b = 4 * threadIdx.x; b < b0; b += 4 * PERM_THREADS) {
+        const float4 v = *reinterpret_cast<const float4 *>(smem_raw + b * sizeof(T));
+        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                     :: "l"(out + b), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+      }
+    }
+  }
+  for (uint32_t b = b0 + threadIdx.x; b < m; b += PERM_THREADS) {
+    const T v = private_bin<OP, T>(smem_raw, m, b);
+    if (to_bits(v) != to_bits(idT)) atomic_combine<OP, T>(out + b, v);
+  }
 }
 
 // Privatised permute into cluster-distributed shared memory.  CL CTAs form a
@@ -236,152 +612,9 @@ __global__ void __launch_bounds__(1024, 1) permute_cluster(PermArgs a, int per) 
   }
 }
 
-// Privatised permute, split by ownership instead of remote atomics: the CL
-// CTAs of a cluster all read the SAME slice of the input (co-scheduled, so
-// L2 serves all but the first read of each line) and each applies only the
-// updates to the bins it owns, with local shared-memory atomics.
-template <int OP, class T, int LOG_CL>
-__global__ void __launch_bounds__(1024, 1) permute_split(PermArgs a, int per) {
-  constexpr int CL = 1 << LOG_CL;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T *bins = reinterpret_cast<T *>(smem_raw);
-  const uint32_t rank = CL > 1 ? cg::this_cluster().block_rank() : 0u;
-  const T idT = Prim<OP, T>::id();
-  for (int b = threadIdx.x; b < per; b += blockDim.x) bins[b] = idT;
-  __syncthreads();
-  const T *src = static_cast<const T *>(a.src);
-  const T c = from_bits<T>(a.cval);
-  const uint32_t m = (uint32_t)a.m;
-  bool bad = false;
-  auto one = [&](int32_t j, T x) {
-    if (j < 0) return;
-    if ((uint32_t)j >= m) { bad = true; return; }
-    if (((uint32_t)j & (CL - 1)) != rank) return;
-    atomic_combine<OP, T>(bins + ((uint32_t)j >> LOG_CL), x);
-  };
-  // Thread index within the cluster's share of the grid.
-  const int64_t cluster_id = blockIdx.x >> LOG_CL;
-  const int64_t nclusters = gridDim.x >> LOG_CL;
-  const int64_t tid = cluster_id * blockDim.x + threadIdx.x;
-  const int64_t nth = nclusters * blockDim.x;
-  if (!a.idx64 && !a.has_src && (reinterpret_cast<uintptr_t>(a.idx) & 15u) == 0) {
-    const int64_t nv = a.n / 4;
-    const uint4 *iv = static_cast<const uint4 *>(a.idx);
-    const int64_t rounds = (nv + 4 * nth - 1) / (4 * nth);
-    for (int64_t r = 0; r < rounds; ++r) {
-      uint4 q[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t v = (r * 4 + u) * nth + tid;
-        q[u] = v < nv ? __ldcg(iv + v) : make_uint4(~0u, ~0u, ~0u, ~0u);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        one((int32_t)q[u].x, c); one((int32_t)q[u].y, c); one((int32_t)q[u].z, c); one((int32_t)q[u].w, c);
-      }
-    }
-    const int64_t tail = a.n - nv * 4;
-    if (tid < tail) one(static_cast<const int32_t *>(a.idx)[nv * 4 + tid], c);
-  } else {
-    for (int64_t i = tid; i < a.n; i += nth) {
-      const int64_t j = perm_idx(a, i);
-      if (j >= (int64_t)m) { bad = true; continue; }
-      one((int32_t)j, a.has_src ? src[i] : c);
-    }
-  }
-  if (bad && rank == 0) raise_error(a.err, DEV_ERR_INDEX);
-  __syncthreads();
-  T *out = static_cast<T *>(a.out);
-  for (int b = threadIdx.x; b < per; b += blockDim.x) {
-    const T v = bins[b];
-    const int64_t j = ((int64_t)b << LOG_CL) | rank;
-    if (v != idT && j < a.m) atomic_combine<OP, T>(out + j, v);
-  }
-}
-
-// Histogram (+ of a small positive constant) with 16-bit counters packed two
-// to a word, so 2^16 bins fit in one CTA's shared memory and every update is
-// local.  Word w holds bin w (low half) and bin w + half (high half), half =
-// ceil(m / 2): neighbouring bins, which skewed (Zipf-like) indices make hot
-// together, sit in different words and banks, so their updates do not
-// serialise on one address.  A counter that wraps is repaired exactly: the
-// carry that ran into the word's other counter is taken back and 65536 is
-// added to the target bin in global memory.
-template <bool AGG>
-__global__ void __launch_bounds__(1024, 1) permute_hist16(PermArgs a) {
-  extern __shared__ __align__(16) uint32_t words[];
-  const uint32_t m = (uint32_t)a.m;
-  const uint32_t nwords = (m + 1) / 2;
-  for (uint32_t b = threadIdx.x; b < nwords; b += blockDim.x) words[b] = 0u;
-  __syncthreads();
-  const uint32_t c = (uint32_t)a.cval;
-  uint32_t *out = static_cast<uint32_t *>(a.out);
-  bool bad = false;
-  auto one = [&](int32_t j) {
-    const bool ok = j >= 0 && (uint32_t)j < m;
-    bad |= (j >= 0 && !ok);
-    uint32_t inc = c;
-    bool lead = ok;
-    if constexpr (AGG) {
-      const unsigned grp = __match_any_sync(0xffffffffu, ok ? j : -1);
-      lead = ok && (__ffs(grp) - 1) == (int)(threadIdx.x & 31);
-      inc = c * (uint32_t)__popc(grp);
-    }
-    if (!lead) return;
-    // Each bin's true count is its 16-bit counter plus 65536 for every time the
-    // counter's unbounded value crossed a multiple of 65536.  Every change to
-    // a counter is one atomic whose returned old word shows the crossing:
-    //  * an update of bin j crosses when old16 + inc > 0xffff;
-    //  * a low counter that crosses also carries +1 into the high counter
-    //    (a crossing for bin j+half when the old high half was 0xffff), and
-    //    the carry is then taken back with -1 (a crossing back when the high
-    //    half it finds is 0).  Accounting for all three keeps every bin exact.
-    const bool low = (uint32_t)j < nwords;
-    const uint32_t wi = low ? (uint32_t)j : (uint32_t)j - nwords;
-    const uint32_t sh = low ? 0u : 16u;
-    const uint32_t old = atomicAdd(&words[wi], inc << sh);
-    if (((old >> sh) & 0xffffu) + inc > 0xffffu) {
-      atomicAdd(out + j, 65536u);
-      if (sh == 0) {
-        int d = (old >> 16) == 0xffffu ? 1 : 0;
-        const uint32_t old2 = atomicSub(&words[wi], 1u << 16);
-        d -= (old2 >> 16) == 0u ? 1 : 0;
-        if (d != 0 && (uint32_t)j + nwords < m) atomicAdd(out + j + nwords, (uint32_t)(d * 65536));
-      }
-    }
-  };
-  const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t nth = (int64_t)gridDim.x * blockDim.x;
-  const int64_t nv = a.n / 4;
-  const uint4 *iv = static_cast<const uint4 *>(a.idx);
-  const int64_t rounds = (nv + 4 * nth - 1) / (4 * nth);
-  for (int64_t r = 0; r < rounds; ++r) {
-    uint4 q[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int64_t v = (r * 4 + u) * nth + tid;
-      q[u] = v < nv ? ld_stream16(iv + v) : make_uint4(~0u, ~0u, ~0u, ~0u);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      one((int32_t)q[u].x); one((int32_t)q[u].y); one((int32_t)q[u].z); one((int32_t)q[u].w);
-    }
-  }
-  const int64_t tail = a.n - nv * 4;
-  one(tid < tail ? static_cast<const int32_t *>(a.idx)[nv * 4 + tid] : -1);
-  if (bad) raise_error(a.err, DEV_ERR_INDEX);
-  __syncthreads();
-  for (uint32_t b = threadIdx.x; b < nwords; b += blockDim.x) {
-    const uint32_t w = words[b];
-    if (w & 0xffffu) atomicAdd(out + b, w & 0xffffu);
-    if ((w >> 16) && b + nwords < m) atomicAdd(out + b + nwords, w >> 16);
-  }
-}
-
 // ----------------------------------------------------------------- host side
-// Shared-memory privatisation pays off when there are many more source
-// elements than bins.  Variant choice (tuning knob, default "auto"):
-// ACC_GB300_PERMUTE = auto | cluster | hist16 | global, ACC_GB300_PERMUTE_AGG = 0 | 1.
+// Variant choice (tuning knob, default "auto"): ACC_GB300_PERMUTE = auto |
+// cluster | global, ACC_GB300_PERMUTE_AGG = 0 | 1 (the cluster kernel's).
 static int env_int(const char *name, int dflt) {
   const char *v = getenv(name);
   return v ? atoi(v) : dflt;
@@ -428,10 +661,29 @@ static int launch_permute_cluster(PermArgs a, bool agg, cudaStream_t s) {
   const int per = (int)cdiv_h(a.m, CL);
   const size_t smem = (size_t)per * sizeof(T);
   const int64_t want = cdiv_h(a.n, 1024 * 16);
-  if (LOG_CL == 0 || strcmp(env_str("ACC_GB300_PERMUTE"), "split") == 0)
-    return launch_cluster(permute_split<OP, T, LOG_CL>, CL, 1024, smem, want * CL, s, a, per);
   if (agg) return launch_cluster(permute_cluster<OP, T, LOG_CL, true>, CL, 1024, smem, want, s, a, per);
   return launch_cluster(permute_cluster<OP, T, LOG_CL, false>, CL, 1024, smem, want, s, a, per);
+}
+
+// One of the shared-memory kernels above on `smem` bytes of bins.  CTAs: one
+// per SM, fewer when each would have less than `per_cta` elements to stream,
+// since every CTA fills and folds a whole copy of the bins.
+template <class K>
+static int launch_private(K kern, std::atomic<uint64_t> &attr_done, size_t smem, int64_t per_cta, const PermArgs &a,
+                          cudaStream_t s) {
+  const Device &d = device_info();
+  smem_attrs_once(kern, d.max_smem_optin, attr_done);
+  int64_t grid = cdiv_h(a.n, per_cta);
+  if (grid > d.sms) grid = d.sms;
+  kern<<<(unsigned)grid, PERM_THREADS, smem, s>>>(a);
+  return check_launch();
+}
+
+template <class T, bool I64>
+static int launch_count(const PermArgs &a, bool wide, size_t smem, int64_t per_cta, cudaStream_t s) {
+  static std::atomic<uint64_t> done32{0}, done16{0};
+  return wide ? launch_private(permute_count32<T, I64>, done32, smem, per_cta, a, s)
+              : launch_private(permute_count16<T, I64>, done16, smem, per_cta, a, s);
 }
 
 template <int OP, class T>
@@ -441,35 +693,38 @@ int permute_typed(Workspace *w, PermArgs a, cudaStream_t s) {
   if (a.n == 0) return ACC_OK;
   const char *variant = env_str("ACC_GB300_PERMUTE");
   const bool agg = env_int("ACC_GB300_PERMUTE_AGG", 0) != 0;
-  const bool force_global = strcmp(variant, "global") == 0;
+  const bool force_global = strcmp(variant, "global") == 0, force_cluster = strcmp(variant, "cluster") == 0;
   constexpr bool int32ish = std::is_same<T, int32_t>::value || std::is_same<T, uint32_t>::value;
+  a.vec = aligned16(a.idx) && (!a.has_src || aligned16(a.src));
+  // Private bins in shared memory from four updates per bin on.
+  const bool many = a.m > 0 && a.n >= 4 * a.m;
+  const int64_t smem_cap = d.max_smem_optin - 1024;
+  const int64_t bytes = a.m * (int64_t)sizeof(T);
+  const int64_t per_cta = 1024 * 8;
+  if (many && !force_global && !force_cluster) {
+    if constexpr (OP == ACC_ADD && !is_fp<T>()) {
+      const bool wide = a.m * 4 <= smem_cap;
+      if (!a.has_src && (a.m + 1) / 2 * 4 <= smem_cap) {
+        const size_t smem = (size_t)(wide ? a.m : (a.m + 1) / 2) * 4;
+        return a.idx64 ? launch_count<T, true>(a, wide, smem, per_cta, s)
+                       : launch_count<T, false>(a, wide, smem, per_cta, s);
+      }
+    }
+    if (bytes <= smem_cap) {
+      static std::atomic<uint64_t> done{0};
+      return launch_private(permute_private<OP, T>, done, (size_t)bytes, per_cta, a, s);
+    }
+  }
   if constexpr (int32ish && OP != ACC_MUL) {
     const int64_t cap_bytes = d.max_smem_optin > (200 << 10) ? (192 << 10) : (int64_t)d.max_smem_optin - (8 << 10);
-    const bool many = a.m > 0 && a.n >= 4 * a.m;
-    // 16-bit packed counters: + of a small positive constant, Int32 indices.
-    const uint32_t c = (uint32_t)a.cval;
-    const bool hist16_ok = OP == ACC_ADD && !a.has_src && !a.idx64 && c > 0 && c < 2048 &&
-                           (reinterpret_cast<uintptr_t>(a.idx) & 15u) == 0 && (a.m + 1) / 2 * 4 <= cap_bytes;
-    const bool want_hist16 = strcmp(variant, "hist16") == 0 ||
-                             (strcmp(variant, "auto") == 0 && a.m * (int64_t)sizeof(T) > cap_bytes);
-    if (!force_global && many && hist16_ok && want_hist16) {
-      const size_t smem = (size_t)((a.m + 1) / 2) * 4;
-      auto kern = agg ? permute_hist16<true> : permute_hist16<false>;
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      int64_t grid = cdiv_h(a.n, 1024 * 16);
-      if (grid > d.sms) grid = d.sms;
-      kern<<<(unsigned)grid, 1024, smem, s>>>(a);
-      return check_launch();
-    }
-    int64_t cap = cap_bytes / (int64_t)sizeof(T);
+    const int64_t cap = cap_bytes / (int64_t)sizeof(T);
     if (!force_global && many) {
-      if (a.m <= cap) return launch_permute_cluster<OP, T, 0>(a, agg, s);
       if (a.m <= 2 * cap) return launch_permute_cluster<OP, T, 1>(a, agg, s);
       if (a.m <= 4 * cap) return launch_permute_cluster<OP, T, 2>(a, agg, s);
       if (a.m <= 8 * cap) return launch_permute_cluster<OP, T, 3>(a, agg, s);
     }
   }
-  int64_t blocks = cdiv_h(a.n, 256);
+  int64_t blocks = cdiv_h(a.vec ? cdiv_h(a.n, 4) : a.n, 256);
   if (blocks > (int64_t)d.sms * 16) blocks = (int64_t)d.sms * 16;
   permute_global<OP, T><<<(unsigned)blocks, 256, 0, s>>>(a);
   return check_launch();
