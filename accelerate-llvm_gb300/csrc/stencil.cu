@@ -5,21 +5,23 @@
 // output, every tap a separate global load, no shared-memory reuse) and
 // 2*rank `stencil_border` kernels on forked streams
 // (accelerate-llvm-ptx/src/Data/Array/Accelerate/LLVM/PTX/Execute.hs:686-776,
-// PTX/CodeGen/Stencil.hs:113-179).  Here one launch covers the whole array:
-// each CTA pulls a (TH + 2R) x (TW + 2PX) halo tile into shared memory with
-// one 2-D TMA load (the x start rounded out to a 16-byte boundary), CTAs
-// whose halo leaves the array overwrite the out-of-range cells with the
+// PTX/CodeGen/Stencil.hs:113-179).  Here one launch covers the whole array.
+// The usual patterns (3x3, 1x3, 3x1, 5x5) stream the rows of a strip of
+// columns through a warp's registers (stencil_rows_kernel).  The others, and
+// the second pass of stencil2, pull a (TH + 2R) x (TW + 2PX) halo tile per CTA
+// into shared memory with one 2-D TMA load (the x start rounded out to a
+// 16-byte boundary), overwrite the cells outside of the array with the
 // boundary rule (accelerate-llvm/src/Data/Array/Accelerate/LLVM/CodeGen/
-// Stencil.hs:195-253), and each thread sweeps a column of TH/4 outputs,
-// keeping one accumulator per output and visiting the taps in the
-// reference's order (rows outer, -r..r; CodeGen/Stencil.hs:73-180).
+// Stencil.hs:195-253), and each thread sweeps a column of outputs, keeping one
+// accumulator per output and visiting the taps in the reference's order
+// (rows outer, -r..r; CodeGen/Stencil.hs:73-180).
 //
 // Arithmetic: acc starts at the additive identity (-0.0) and every tap is one
 // fused multiply-add, acc = fma(w, x, acc), in tap order, so Float32 / Float64
 // results are bit-identical to a sequential C evaluation with C99 fma()
 // (correctly rounded).  Taps whose weight is exactly zero are not part of the
 // pattern and are not read.
-#include "stencil_common.cuh"
+#include "stencil_rows.cuh"
 
 namespace accgb {
 
@@ -244,160 +246,6 @@ stencil_fast_kernel(const __grid_constant__ CUtensorMap tin, StencilArgs a, Sten
   }
 }
 
-// ----------------------------------------------------------------- persistent pipeline
-// The specialised sweep run by persistent CTAs over a static tile schedule
-// (tile = blockIdx.x + k * gridDim.x, row-major over the tile grid): the halo
-// tile of tile k+2 is loading (TMA) while tile k is computed, and each output
-// tile leaves through a TMA store from shared memory, clipped at the array's
-// edge by the copy engine.  Used for 16-byte aligned, non-accumulating calls.
-template <class T, int RY, int RX, int PAT>
-__global__ void __launch_bounds__(ST_THREADS, (sizeof(T) == 4 && RY * RX <= 1) ? 3 : 1)
-stencil_pipe_kernel(const __grid_constant__ CUtensorMap tin, const __grid_constant__ CUtensorMap tout,
-                    StencilArgs a, StencilW<T> W, uint32_t zmask_lo, uint32_t zmask_hi, int ntx, int64_t ntiles) {
-  constexpr int PX = ((RX * (int)sizeof(T) + 15) / 16) * 16 / (int)sizeof(T);
-  constexpr int SW = SF_TW + 2 * PX;
-  constexpr int SH = SF_TH + 2 * RY;
-  constexpr int KW = 2 * RX + 1;
-  constexpr int NT = (2 * RY + 1) * KW;
-  constexpr int IN_BYTES = ((SW * SH * (int)sizeof(T)) + 127) / 128 * 128;
-  constexpr int OUT_BYTES = SF_TW * SF_TH * (int)sizeof(T);
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  auto inb = [&](int s) { return reinterpret_cast<T *>(base + s * IN_BYTES); };
-  auto outb = [&](int s) { return reinterpret_cast<T *>(base + 2 * IN_BYTES + s * OUT_BYTES); };
-  __shared__ uint64_t full[2];
-  __shared__ int s_abort;
-  const int tid = threadIdx.x;
-  const T *in = static_cast<const T *>(a.in);
-
-  auto issue = [&](int s, int64_t tile) {  // thread 0
-    const int64_t ty = tile / ntx, tx = tile % ntx;
-    mbar_expect_tx(&full[s], SW * SH * sizeof(T));
-    tma_load_2d(inb(s), &tin, (int)(tx * SF_TW - PX), (int)(ty * SF_TH - RY), &full[s]);
-  };
-  if (tid == 0) {
-    prefetch_tmap(&tin);
-    prefetch_tmap(&tout);
-    s_abort = 0;
-    mbar_init(&full[0], 1);
-    mbar_init(&full[1], 1);
-    fence_mbar_init();
-    if ((int64_t)blockIdx.x < ntiles) issue(0, blockIdx.x);
-    if ((int64_t)blockIdx.x + gridDim.x < ntiles) issue(1, (int64_t)blockIdx.x + gridDim.x);
-  }
-  __syncthreads();
-
-  T w[NT];
-#pragma unroll
-  for (int k = 0; k < NT; ++k) w[k] = W.w[k];
-  const int col = tid % SF_TW;
-  const int oy0 = (tid / SF_TW) * SF_ROWS;
-
-  for (int k = 0;; ++k) {
-    const int64_t tile = (int64_t)blockIdx.x + (int64_t)k * gridDim.x;
-    if (tile >= ntiles) break;
-    const int s = k & 1;
-    const int64_t ty = tile / ntx, tx = tile % ntx;
-    const int64_t tx0 = tx * SF_TW, ty0 = ty * SF_TH;
-    const int64_t gx0 = tx0 - PX, gy0 = ty0 - RY;
-    // A tile that never lands sets s_abort; the CTA stops at the next
-    // barrier, before it stores from or loads into its buffers (no extra
-    // barrier per tile).
-    if (!mbar_wait_flagged(&full[s], (uint32_t)(k >> 1) & 1u, a.err)) s_abort = 1;
-    T *tile_in = inb(s);
-    if (gx0 < 0 || gy0 < 0 || gx0 + SW > a.in_w || gy0 + SH > a.in_h) {
-      for (int q = tid; q < SW * SH; q += ST_THREADS) {
-        const int sy = q / SW, sx = q % SW;
-        const int64_t gy = gy0 + sy, gx = gx0 + sx;
-        if (gy >= 0 && gy < a.in_h && gx >= 0 && gx < a.in_w) continue;
-        tile_in[sy * SW + sx] = a.boundary == ACC_CONSTANT
-                                    ? from_bits<T>(a.cval)
-                                    : in[bound_index(gy, a.in_h, a.boundary) * a.in_pitch + bound_index(gx, a.in_w, a.boundary)];
-      }
-      __syncthreads();
-    }
-    T acc[SF_ROWS];
-#pragma unroll
-    for (int r = 0; r < SF_ROWS; ++r) acc[r] = Prim<ACC_ADD, T>::id();
-    const T *trow = tile_in + oy0 * SW + PX + col;
-#pragma unroll
-    for (int ir = 0; ir < SF_ROWS + 2 * RY; ++ir) {
-      T xv[KW];
-#pragma unroll
-      for (int dx = 0; dx < KW; ++dx) xv[dx] = trow[ir * SW + dx - RX];
-#pragma unroll
-      for (int dyi = 0; dyi < 2 * RY + 1; ++dyi) {
-        const int r = ir - dyi;
-        if (r < 0 || r >= SF_ROWS) continue;
-#pragma unroll
-        for (int dx = 0; dx < KW; ++dx) {
-          const int q = dyi * KW + dx;
-          if constexpr (PAT == 1) {
-            if (q == 0 || q == 2 || q == 6 || q == 8) continue;
-          }
-          if constexpr (PAT == 2) {
-            const bool zero = q < 32 ? ((zmask_lo >> q) & 1u) : ((zmask_hi >> (q - 32)) & 1u);
-            if (zero) continue;
-          }
-          acc[r] = fma_tap(w[q], xv[dx], acc[r]);
-        }
-      }
-    }
-    // The store issued from this output buffer two tiles ago must have read it.
-    if (tid == 0 && k >= 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-    __syncthreads();
-    if (s_abort) {
-      // bounded waits for this tile's load and the next one, issued into the
-      // other stage, then stop (stores already issued complete below)
-      if (tid == 0) {
-        mbar_wait(&full[s], (uint32_t)(k >> 1) & 1u);
-        if (tile + (int64_t)gridDim.x < ntiles) mbar_wait(&full[s ^ 1], (uint32_t)((k + 1) >> 1) & 1u);
-      }
-      break;
-    }
-    T *ob = outb(s);
-#pragma unroll
-    for (int r = 0; r < SF_ROWS; ++r) ob[(oy0 + r) * SF_TW + col] = acc[r];
-    fence_proxy_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      tma_store_2d(&tout, (int)tx0, (int)ty0, ob);
-      tma_store_commit();
-      const int64_t next = tile + 2 * (int64_t)gridDim.x;
-      if (next < ntiles) issue(s, next);  // every thread is done with inb[s]
-    }
-  }
-  if (tid == 0) tma_store_wait_all();
-}
-
-template <class T, int RY, int RX, int PAT>
-int stencil_pipe_launch(StencilArgs a, const StencilW<T> &W, uint32_t zlo, uint32_t zhi, cudaStream_t s,
-                        const CUtensorMap &tin, const CUtensorMap &tout) {
-  constexpr int PX = ((RX * (int)sizeof(T) + 15) / 16) * 16 / (int)sizeof(T);
-  constexpr int SW = SF_TW + 2 * PX;
-  constexpr int SH = SF_TH + 2 * RY;
-  constexpr int IN_BYTES = ((SW * SH * (int)sizeof(T)) + 127) / 128 * 128;
-  constexpr int OUT_BYTES = SF_TW * SF_TH * (int)sizeof(T);
-  const size_t smem = 2 * (size_t)IN_BYTES + 2 * (size_t)OUT_BYTES + 128;
-  auto kern = stencil_pipe_kernel<T, RY, RX, PAT>;
-  static int per_sm = 0;
-  if (per_sm == 0) {
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, ST_THREADS, smem) != cudaSuccess || per_sm < 1) {
-      cudaGetLastError();
-      per_sm = 1;
-    }
-  }
-  const int64_t ntx = cdiv_h(a.w, SF_TW), nty = cdiv_h(a.h, SF_TH);
-  const int64_t ntiles = ntx * nty;
-  if (ntx > (1 << 30) || nty > (1 << 30)) return ACC_ERR_TOO_LARGE;
-  int64_t grid = (int64_t)device_info().sms * per_sm;
-  if (grid > ntiles) grid = ntiles;
-  kern<<<(unsigned)grid, ST_THREADS, smem, s>>>(tin, tout, a, W, zlo, zhi, (int)ntx, ntiles);
-  return check_launch();
-}
-
 template <class T, int RY, int RX, int PAT>
 int stencil_fast_launch(StencilArgs a, const StencilW<T> &W, uint32_t zlo, uint32_t zhi, cudaStream_t s) {
   constexpr int PX = ((RX * (int)sizeof(T) + 15) / 16) * 16 / (int)sizeof(T);
@@ -408,13 +256,6 @@ int stencil_fast_launch(StencilArgs a, const StencilW<T> &W, uint32_t zlo, uint3
   memset(&tin, 0, sizeof(tin));
   a.tma = encode_2d(&tin, a.in, sizeof(T), (uint64_t)a.in_w, (uint64_t)a.in_h, (uint64_t)a.in_pitch * sizeof(T),
                     SW, SH, false);
-  if (a.tma && !a.accumulate) {
-    CUtensorMap tout;
-    memset(&tout, 0, sizeof(tout));
-    if (encode_2d(&tout, a.out, sizeof(T), (uint64_t)a.w, (uint64_t)a.h, (uint64_t)a.out_pitch * sizeof(T), SF_TW,
-                  SF_TH, false))
-      return stencil_pipe_launch<T, RY, RX, PAT>(a, W, zlo, zhi, s, tin, tout);
-  }
   auto kern = stencil_fast_kernel<T, RY, RX, PAT>;
   static std::atomic<uint64_t> attr_done{0};
   smem_attrs_once(kern, (int)smem, attr_done, false);
@@ -422,6 +263,173 @@ int stencil_fast_launch(StencilArgs a, const StencilW<T> &W, uint32_t zlo, uint3
   if (gy > 65535 || gx > (1ll << 31) - 1) return ACC_ERR_TOO_LARGE;
   kern<<<dim3((unsigned)gx, (unsigned)gy), ST_THREADS, smem, s>>>(tin, a, W, zlo, zhi);
   return check_launch();
+}
+
+// ----------------------------------------------------------------- row streaming
+// Every call but the second pass of stencil2, radii up to 2 as instantiated
+// below.  A warp owns a strip of 32 x E columns and SR_ROWS output rows, and
+// reads the input rows of its range in increasing order straight into
+// registers, `ahead` rows ahead; a row's neighbours left and right come from
+// the other lanes by shuffle, and each lane keeps the accumulators of the
+// 2 RY + 1 output rows that an input row is a tap row of, rotating by the
+// unrolled row loop.  No shared memory and no barrier: a warp waits only for
+// its own loads.  Every output accumulates its taps rows outer, then columns,
+// one fused multiply-add each.  Warps whose halo leaves the array take their
+// rows through the boundary rule, one at a time.
+//
+// Bound: HBM (3x3), issue (5x5).  Measured on a GB300, Float32 8192 x 8192
+// (floor 79 us) against halo tiles through shared memory in a two-stage TMA
+// pipeline with barriers (and, for 8191 x 8191, which TMA cannot describe, one
+// tile per CTA read element by element): 3x3 108 -> 86 us, 5x5 153 -> 129 us;
+// 8191 x 8191 360 -> 101 us and 644 -> 164 us.
+// Few rows per warp: neighbouring warps then work on neighbouring rows, which
+// DRAM and L2 reward (3x3: 10 rows 86 us, 20 rows 90, 64 rows 117, 144 rows --
+// whole waves of warps -- 147), against the 2 RY rows that adjacent warps
+// both read.  Two warps per CTA, so that a slot is refilled as soon as they end
+// (256 threads: 95 us at 16 rows against 90).  Registers: 72 (14 CTAs per SM)
+// for 16-byte rows; the strided form needs 91 (10) and takes 9 rows ahead (6
+// rows ahead: 105 us).  Float32 taps in pairs (fma.rn.f32x2) were slower (129
+// us): the weights then live in registers, twice.
+constexpr int SR_THREADS = 64;
+template <int RY, bool VEC> constexpr int sr_ahead() { return RY == 0 ? 4 : RY == 2 ? 5 : VEC ? 6 : 9; }  // of 2 RY + 1
+template <class T, int RY, bool VEC> constexpr int sr_ctas() {  // 8-byte types: registers without spills
+  return sizeof(T) == 8 ? (RY == 2 ? 5 : 8) : RY == 2 ? 8 : VEC ? 14 : 10;
+}
+// 8-byte types are bound by their multiply-adds, of which the rows that two warps share cost some twice
+template <class T, int RY, bool VEC> constexpr int sr_rows() {
+  return sizeof(T) == 8 ? (RY == 2 ? 96 : 32) : RY == 2 ? 20 : VEC ? 10 : 12;
+}
+
+// One input row (window `win`) applied to the accumulators, whose roles start
+// at slot I: output row r - RY + k takes input row r as its tap row 2 RY - k.
+template <class T, int RY, int RX, int PAT, int I, int E>
+__device__ __forceinline__ void rows_apply(const StencilW<T> &W, uint32_t zmask, const T (&win)[2 * RX + 1][E],
+                                           T (&acc)[2 * RY + 1][E]) {
+  constexpr int K = 2 * RY + 1, KW = 2 * RX + 1;
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+#pragma unroll
+    for (int dx = 0; dx < KW; ++dx) {
+      const int q = (2 * RY - k) * KW + dx;
+      if constexpr (PAT == 1) {
+        if (q == 0 || q == 2 || q == 6 || q == 8) continue;
+      }
+      if constexpr (PAT == 2) {
+        if ((zmask >> q) & 1u) continue;
+      }
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[(k + I) % K][e] = fma_tap(W.w[q], win[dx][e], acc[(k + I) % K][e]);
+    }
+}
+// f(std::integral_constant<int, 0>()) ... f(N - 1) until f returns false.
+template <int N, int I = 0, class F> __device__ __forceinline__ bool rows_unroll(F &&f) {
+  if constexpr (I < N) {
+    if (!f(std::integral_constant<int, I>())) return false;
+    return rows_unroll<N, I + 1>(f);
+  } else {
+    return true;
+  }
+}
+
+template <class T, int RY, int RX, int PAT, bool VEC>
+__global__ void __launch_bounds__(SR_THREADS, sr_ctas<T, RY, VEC>())
+stencil_rows_kernel(const __grid_constant__ StencilArgs a, const __grid_constant__ StencilW<T> W, uint32_t zmask,
+                    int64_t strips, int rows) {
+  using S = Strip<T, RX, VEC>;
+  using Row = typename S::Row;
+  constexpr int E = S::E, K = 2 * RY + 1, KW = 2 * RX + 1, D = sr_ahead<RY, VEC>();
+  static_assert(D % K == 0, "the accumulators' roles rotate with the unrolled loop");
+  const int64_t gw = (int64_t)blockIdx.x * (SR_THREADS / 32) + (threadIdx.x >> 5);
+  const int64_t x0 = gw % strips * (32 * E), y0 = gw / strips * rows;
+  if (y0 >= a.h) return;
+  const int64_t y1 = y0 + rows < a.h ? y0 + rows : a.h;
+  S strip;
+  strip.init(x0, a.in_w, a.boundary, from_bits<T>(a.cval));
+  T acc[K][E];
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+#pragma unroll
+    for (int e = 0; e < E; ++e) acc[k][e] = Prim<ACC_ADD, T>::id();
+  const int n = (int)(y1 - y0) + 2 * RY;  // input rows y0 - RY ..; output row y0 + t - 2 RY is complete after row t
+  T *o = static_cast<T *>(a.out) + (y0 - 2 * RY) * a.out_pitch;
+  if (x0 >= RX && x0 + 32 * E + RX <= a.in_w && y0 >= RY && y1 + RY <= a.in_h) {
+    const T *first = static_cast<const T *>(a.in) + (y0 - RY) * a.in_pitch;
+    const T *p = first + strip.inner_column(x0), *h = first + strip.inner_halo(x0);
+    Row ring[D];
+#pragma unroll
+    for (int i = 0; i < D; ++i)
+      if (i < n) {
+        strip.load_inner(p, h, ring[i]);
+        p += a.in_pitch;
+        h += a.in_pitch;
+      }
+    for (int t0 = 0; t0 < n; t0 += D) {
+      const bool go = rows_unroll<D>([&](auto ic) -> bool {
+        constexpr int I = decltype(ic)::value;
+        const int t = t0 + I;
+        if (t >= n) return false;
+        T win[KW][E];
+        strip.window(ring[I], win);
+        if (t + D < n) {
+          strip.load_inner(p, h, ring[I]);
+          p += a.in_pitch;
+          h += a.in_pitch;
+        }
+        rows_apply<T, RY, RX, PAT, I % K, E>(W, zmask, win, acc);
+        if (t >= 2 * RY) strip.store(o, x0, a.w, acc[I % K]);
+        o += a.out_pitch;
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[I % K][e] = Prim<ACC_ADD, T>::id();
+        return true;
+      });
+      if (!go) break;
+    }
+    return;
+  }
+  for (int t0 = 0; t0 < n; t0 += K) {
+    const bool go = rows_unroll<K>([&](auto ic) -> bool {
+      constexpr int I = decltype(ic)::value;
+      const int t = t0 + I;
+      if (t >= n) return false;
+      const int64_t r = y0 - RY + t;
+      const bool yin = r >= 0 && r < a.in_h;
+      Row row;
+      if (!yin && a.boundary == ACC_CONSTANT) strip.fill(row);
+      else strip.load(static_cast<const T *>(a.in) + (yin ? r : bound_index(r, a.in_h, a.boundary)) * a.in_pitch, row);
+      T win[KW][E];
+      strip.window(row, win);
+      rows_apply<T, RY, RX, PAT, I, E>(W, zmask, win, acc);
+      if (t >= 2 * RY) strip.store(o, x0, a.w, acc[I]);
+      o += a.out_pitch;
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[I][e] = Prim<ACC_ADD, T>::id();
+      return true;
+    });
+    if (!go) break;
+  }
+}
+
+template <class T, int RY, int RX, int PAT, bool VEC>
+static int stencil_rows_on(const StencilArgs &a, const StencilW<T> &W, uint32_t zmask, cudaStream_t s) {
+  constexpr int WARPS = SR_THREADS / 32;
+  const int64_t strips = cdiv_h(a.w, 32 * (16 / (int)sizeof(T)));
+  // Fewer rows per warp where the array would not fill the machine with warps.
+  const int64_t resident = (int64_t)device_info().sms * sr_ctas<T, RY, VEC>() * WARPS;
+  int64_t rows = cdiv_h(strips * a.h, resident);
+  if (rows > sr_rows<T, RY, VEC>()) rows = sr_rows<T, RY, VEC>();
+  const int64_t grid = cdiv_h(strips * cdiv_h(a.h, rows), WARPS);
+  if (grid > 0x7fffffffll) return ACC_ERR_TOO_LARGE;
+  stencil_rows_kernel<T, RY, RX, PAT, VEC><<<(unsigned)grid, SR_THREADS, 0, s>>>(a, W, zmask, strips, (int)rows);
+  return check_launch();
+}
+template <class T, int RY, int RX, int PAT>
+static int stencil_rows_launch(const StencilArgs &a, const StencilW<T> &W, uint32_t zmask, cudaStream_t s) {
+  // 16-byte loads and stores: every row of both arrays starts on a 16-byte boundary.
+  constexpr int E = 16 / (int)sizeof(T);
+  const bool vec = aligned16(a.in) && aligned16(a.out) && a.w % E == 0 && a.in_w % E == 0 && a.in_pitch % E == 0 &&
+                   a.out_pitch % E == 0;
+  return vec ? stencil_rows_on<T, RY, RX, PAT, true>(a, W, zmask, s)
+             : stencil_rows_on<T, RY, RX, PAT, false>(a, W, zmask, s);
 }
 
 // Zero-weight mask of the taps (bit k set: weight k is zero).
@@ -437,12 +445,19 @@ void zero_mask(const StencilW<T> &W, int n, uint32_t &lo, uint32_t &hi) {
 template <class T, int RY, int RX>
 int stencil_fast_pat(StencilArgs a, const StencilW<T> &W, cudaStream_t s) {
   constexpr int NT = (2 * RY + 1) * (2 * RX + 1);
+  static_assert(NT <= 32, "one mask word");
   uint32_t lo, hi;
   zero_mask(W, NT, lo, hi);
-  if (lo == 0 && hi == 0) return stencil_fast_launch<T, RY, RX, 0>(a, W, 0, 0, s);
-  if (RY == 1 && RX == 1 && lo == ((1u << 0) | (1u << 2) | (1u << 6) | (1u << 8)))
-    return stencil_fast_launch<T, RY, RX, 1>(a, W, 0, 0, s);
-  return stencil_fast_launch<T, RY, RX, 2>(a, W, lo, hi, s);
+  auto pattern = [&](auto pat) {
+    constexpr int PAT = decltype(pat)::value;
+    return a.accumulate ? stencil_fast_launch<T, RY, RX, PAT>(a, W, lo, 0, s)
+                        : stencil_rows_launch<T, RY, RX, PAT>(a, W, lo, s);
+  };
+  if (lo == 0) return pattern(IC<0>{});
+  if constexpr (RY == 1 && RX == 1) {
+    if (lo == ((1u << 0) | (1u << 2) | (1u << 6) | (1u << 8))) return pattern(IC<1>{});
+  }
+  return pattern(IC<2>{});
 }
 
 // ----------------------------------------------------------------- host side
