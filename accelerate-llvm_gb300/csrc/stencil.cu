@@ -413,10 +413,11 @@ template <class T, int RY, int RX, int PAT, bool VEC>
 static int stencil_rows_on(const StencilArgs &a, const StencilW<T> &W, uint32_t zmask, cudaStream_t s) {
   constexpr int WARPS = SR_THREADS / 32;
   const int64_t strips = cdiv_h(a.w, 32 * (16 / (int)sizeof(T)));
-  // Fewer rows per warp where the array would not fill the machine with warps.
+  // Whole waves of resident warps, as few as keep a warp's rows within sr_rows
+  // (one wave, and fewer rows, where the array is small).
   const int64_t resident = (int64_t)device_info().sms * sr_ctas<T, RY, VEC>() * WARPS;
-  int64_t rows = cdiv_h(strips * a.h, resident);
-  if (rows > sr_rows<T, RY, VEC>()) rows = sr_rows<T, RY, VEC>();
+  const int64_t waves = cdiv_h(strips * a.h, resident * sr_rows<T, RY, VEC>());
+  const int64_t rows = cdiv_h(strips * a.h, resident * waves);
   const int64_t grid = cdiv_h(strips * cdiv_h(a.h, rows), WARPS);
   if (grid > 0x7fffffffll) return ACC_ERR_TOO_LARGE;
   stencil_rows_kernel<T, RY, RX, PAT, VEC><<<(unsigned)grid, SR_THREADS, 0, s>>>(a, W, zmask, strips, (int)rows);

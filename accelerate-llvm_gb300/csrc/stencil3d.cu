@@ -85,34 +85,42 @@ stencil3d_kernel(const __grid_constant__ Stencil3Args a, const __grid_constant__
   }
 }
 
-// The 2.5-D plane-streaming form, for 3x3x3 patterns: a CTA owns a 32 x 32
-// tile of columns and rows and a range of planes, and streams the planes of
-// its tile's halo through a ring of S3S_STAGES shared-memory buffers in
-// increasing order, S3S_STAGES - 1 planes loading (cp.async, no registers
+// The 2.5-D plane-streaming form, for 3x3x3 patterns: a CTA owns a tile of 64
+// (8-byte types: 32) columns and 16 rows and a range of planes, and streams the
+// planes of its tile's halo through a ring of 3 (8-byte types: 4) shared-memory
+// buffers in increasing order, all but one loading (cp.async, no registers
 // held) while one is used.  A plane contributes to the 3 outputs it is a tap
-// plane of; each thread keeps those outputs' accumulators for its 4 rows in
-// registers and rotates them as the planes go by, so the output of plane z is
-// complete (and stored) once plane z+1 has been applied.  Every plane is read
-// from DRAM once per tile (plus a 2-plane overlap between a CTA's plane range
-// and its neighbours') and from shared memory 3 rows per output row.  The
-// planes arrive in increasing order, so each output still accumulates its
-// taps planes outer, then rows, then columns, one fused multiply-add each,
-// exactly as the direct kernel and the oracle do.
+// plane of; each thread keeps those outputs' accumulators for 4 rows of 2 (1)
+// adjacent columns in registers; they move up as the planes go by (the loop is
+// unrolled three times, so that moving them costs nothing), so the output of
+// plane z is complete (and stored) once plane z+1 has been applied.  Every
+// plane is read from DRAM once per tile (plus a 2-plane overlap between a CTA's
+// plane range and its neighbours').  The planes arrive in increasing order, so
+// each output still accumulates its taps planes outer, then rows, then
+// columns, one fused multiply-add each, exactly as the direct kernel and the
+// oracle do.
 //
-// A buffer row holds columns x0-PX .. x0+32+PX-1 (PX = 16 bytes of elements,
-// so each row starts on a 16-byte boundary); rows whose columns all lie in
-// the array are copied in 16-byte pieces when the array's rows are 16-byte
-// aligned, the rest element by element with each index remapped by the
-// boundary (constant-boundary cells outside the array are written directly).
+// A buffer row holds columns x0-PX .. x0+TW+PX-1 (PX = 16 bytes of elements,
+// so each row starts on a 16-byte boundary), copied in 16-byte pieces when the
+// array's rows are 16-byte aligned, else element by element; outside of the
+// array only columns -1 and w are read, each from its remapped place, and
+// cells under the constant boundary are written once.
 // PAT selects the taps at compile time: 0 = all 27 weights non-zero, 1 = the
 // 7-point star (centre and the six face neighbours), 2 = any pattern (each tap
 // tested against a mask of the non-zero weights).
-// Output rows per thread: 4 (a tile of 32 x 32 outputs).  Measured on a
-// GB300, 512^3 Float32: 8 rows per thread (80 registers, 3 CTAs per SM)
-// 0.43 ms against 0.38 ms for 4 rows (64 registers, 4 CTAs per SM).
-constexpr int S3S_TX = 32, S3S_TY = 8, S3S_ROWS = 4, S3S_STAGES = 4;
+//
+// Bound: issue and the FP32 pipe (27 multiply-adds per output), then HBM.
+// Measured on a GB300, 512^3 Float32 (floor 158 us): 365 -> 213 us, star 295 ->
+// 189; 511^3 513 -> 281.  What gave it: copying the three unused halo columns
+// of edge tiles with a remap per element cost 420 instructions per plane in a
+// quarter of the warps (361 -> 240 us without it); two columns per thread
+// 253 -> 240; 128 threads per CTA and the unrolled loop 213.  Four stages 218
+// (and 209 for the star: more planes in flight leave L2 sooner), 8 rows per thread
+// 220, packed multiply-adds (fma.rn.f32x2) 278: they run at half rate.
+constexpr int S3S_TX = 32, S3S_TY = 4, S3S_ROWS = 4;
 constexpr int S3S_OY = S3S_TY * S3S_ROWS;  // output rows per tile
 constexpr int S3S_THREADS = S3S_TX * S3S_TY;
+template <class T> constexpr int s3_stages() { return sizeof(T) == 4 ? 3 : 4; }
 
 __device__ __forceinline__ void cp_async_16(void *dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
@@ -131,125 +139,166 @@ template <int PAT> __device__ __forceinline__ bool s3_tap(int t, uint32_t mask) 
   else return (mask >> t) & 1u;
 }
 
+template <class T> constexpr int s3_cols() { return sizeof(T) == 4 ? 2 : 1; }  // adjacent output columns per thread
+template <class T> constexpr int s3_ctas() { return sizeof(T) == 4 ? 6 : 4; }
+
 template <class T, int PAT>
-__global__ void __launch_bounds__(S3S_THREADS, sizeof(T) == 4 ? 4 : 2)
+__global__ void __launch_bounds__(S3S_THREADS, s3_ctas<T>())
 stencil3d_stream_kernel(const __grid_constant__ Stencil3Args a, const __grid_constant__ Stencil3W<T> W,
                         int64_t zchunk, uint32_t mask, int vec) {
-  constexpr int R = 1, K = 3;
+  constexpr int R = 1, K = 3, CE = s3_cols<T>();
+  constexpr int S3S_STAGES = s3_stages<T>();
   constexpr int PX = 16 / (int)sizeof(T);             // left/right pad: one 16-byte piece
-  constexpr int PW = S3S_TX + 2 * PX, PH = S3S_OY + 2 * R;
+  constexpr int TW = S3S_TX * CE;                     // output columns per tile
+  constexpr int PW = TW + 2 * PX, PH = S3S_OY + 2 * R;
   constexpr int CPR = PW * (int)sizeof(T) / 16;        // 16-byte pieces per buffer row
   constexpr int EPC = 16 / (int)sizeof(T);             // elements per piece
   constexpr int NPC = (PH * CPR + S3S_THREADS - 1) / S3S_THREADS;  // pieces per thread
   __shared__ __align__(16) T plane[S3S_STAGES][PH][PW];
   const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * S3S_TX + tx;
-  const int64_t x0 = (int64_t)blockIdx.x * S3S_TX, y0 = (int64_t)blockIdx.y * S3S_OY;
+  const int64_t x0 = (int64_t)blockIdx.x * TW, y0 = (int64_t)blockIdx.y * S3S_OY;
   const int64_t z0 = (int64_t)blockIdx.z * zchunk;
   int64_t z1 = z0 + zchunk;
   if (z1 > a.d) z1 = a.d;
   if (z0 >= z1) return;
   const T *in = static_cast<const T *>(a.in);
-  T *out = static_cast<T *>(a.out);
   const T cval = from_bits<T>(a.cval);
   const int b = a.boundary;
   const int64_t gxs = x0 - PX;  // column of buffer column 0
   const int64_t hw = a.h * a.w;
 
   // This thread's pieces, the same in every plane: piece q = tid + u * threads
-  // is buffer row q / CPR, columns (q % CPR) * EPC ...  Mode 0: one 16-byte
-  // copy from element `off` of the plane; 1: element by element from row
-  // offset `off`, each column remapped; 2: constant cells; 3: no piece.
-  int64_t off[NPC];
-  int mode[NPC];
+  // is buffer row q / CPR, columns (q % CPR) * EPC ..., at element q * EPC of a
+  // buffer.  Of the columns outside of the array only -1 and w are read.
+  // cnt: elements of the piece to copy from src (its first one in plane 0):
+  // EPC in one 16-byte copy (vec) or singly, fewer at the right edge; bit 3: and the
+  // element after them from column w's remapped place; bit 4: only the last
+  // element, from src (column -1, remapped).  Constant cells are written here
+  // once: no copy ever overwrites them.
+  constexpr int AFTER = 8, LAST = 16;
+  const T *src[NPC];
+  int cnt[NPC];
+  bool plain = true;
+  const int64_t wr_col = bound_index(a.w, a.w, b);  // where column w reads
 #pragma unroll
   for (int u = 0; u < NPC; ++u) {
     const int q = tid + u * S3S_THREADS;
-    mode[u] = 3;
-    off[u] = 0;
+    cnt[u] = 0;
+    src[u] = in;
     if (q < PH * CPR) {
       const int sy = q / CPR, c = q % CPR;
       const int64_t gy = y0 - R + sy, gx = gxs + (int64_t)c * EPC;
       const bool yin = gy >= 0 && gy < a.h;
-      if (!yin && b == ACC_CONSTANT) {
-        mode[u] = 2;
-      } else {
-        const int64_t row = (yin ? gy : bound_index(gy, a.h, b)) * a.w;
-        const bool whole = vec && gx >= 0 && gx + EPC <= a.w;
-        mode[u] = whole ? 0 : 1;
-        off[u] = whole ? row + gx : row;
+      const T *row = in + (yin ? gy : bound_index(gy, a.h, b)) * a.w;
+      if (yin || b != ACC_CONSTANT) {
+        const int64_t left = a.w - gx;  // columns from gx on
+        if (gx < 0) {  // columns -EPC .. -1
+          cnt[u] = b == ACC_CONSTANT ? 0 : LAST;
+          src[u] = row + bound_index(-1, a.w, b);
+        } else {
+          cnt[u] = left >= EPC ? EPC : left > 0 ? (int)left : 0;
+          if (left >= 0 && left < EPC && b != ACC_CONSTANT) cnt[u] |= AFTER;
+          src[u] = row + gx;
+        }
       }
+      if (b == ACC_CONSTANT) {
+#pragma unroll
+        for (int st = 0; st < S3S_STAGES; ++st)
+#pragma unroll
+          for (int e = 0; e < EPC; ++e)
+            if (!yin || gx + e < 0 || gx + e >= a.w) plane[st][sy][c * EPC + e] = cval;
+      }
+      plain = plain && vec && cnt[u] == EPC;
     }
   }
+  // A tile whose pieces are all 16-byte copies tests no counts.
+  plain = __syncthreads_and(plain);
 
   // Issue the copies of virtual plane p (which may lie outside [0, d)) into
   // buffer `buf`.
-  auto issue = [&](int64_t p, int buf) {
-    const bool pin = p >= 0 && p < a.d;
+  const int d = (int)a.d;
+  auto issue = [&](int p, int buf) {
+    const bool pin = p >= 0 && p < d;
     if (!pin && b == ACC_CONSTANT) {
       for (int q = tid; q < PH * PW; q += S3S_THREADS) plane[buf][q / PW][q % PW] = cval;
       return;
     }
-    const T *pl = in + (pin ? p : bound_index(p, a.d, b)) * hw;
+    const int64_t off = (int64_t)(pin ? p : (int)bound_index(p, d, b)) * hw;
+    T *dst = &plane[buf][0][0] + tid * EPC;
+    if (plain) {
+#pragma unroll
+      for (int u = 0; u < NPC; ++u)
+        if ((u + 1) * S3S_THREADS <= PH * CPR || tid + u * S3S_THREADS < PH * CPR)
+          cp_async_16(dst + u * S3S_THREADS * EPC, src[u] + off);
+      return;
+    }
 #pragma unroll
     for (int u = 0; u < NPC; ++u) {
-      const int q = tid + u * S3S_THREADS;
-      T *dst = &plane[buf][0][0] + (q / CPR) * PW + (q % CPR) * EPC;
-      if (mode[u] == 0) {
-        cp_async_16(dst, pl + off[u]);
-      } else if (mode[u] == 1) {
-        const int64_t gx = gxs + (int64_t)(q % CPR) * EPC;
+      T *to = dst + u * S3S_THREADS * EPC;
+      const T *s = src[u] + off;
+      if (vec && cnt[u] == EPC) {
+        cp_async_16(to, s);
+      } else {
 #pragma unroll
-        for (int e = 0; e < EPC; ++e) {
-          const int64_t x = gx + e;
-          const bool xin = x >= 0 && x < a.w;
-          if (!xin && b == ACC_CONSTANT) dst[e] = cval;
-          else cp_async_el<sizeof(T)>(dst + e, pl + off[u] + (xin ? x : bound_index(x, a.w, b)));
+        for (int e = 0; e < EPC; ++e)
+          if (e < (cnt[u] & 7)) cp_async_el<sizeof(T)>(to + e, s + e);
+        if (cnt[u] & AFTER) {
+          const int n = cnt[u] & 7;
+          const int64_t gx = gxs + (int64_t)((tid + u * S3S_THREADS) % CPR) * EPC;
+          cp_async_el<sizeof(T)>(to + n, s + (wr_col - gx));
+        } else if (cnt[u] & LAST) {
+          cp_async_el<sizeof(T)>(to + EPC - 1, s);
         }
-      } else if (mode[u] == 2) {
-#pragma unroll
-        for (int e = 0; e < EPC; ++e) dst[e] = cval;
       }
     }
   };
 
-  // acc[s][r]: the accumulator of row r of output plane p - R + k lives in
-  // slot s = (k + ROT) % K while plane p is applied; ROT advances by one per
-  // plane, so the finished output's slot becomes the newest output's without
-  // moving registers.
-  T acc[K][S3S_ROWS];
+  // acc[k][r][c]: the accumulator of row r, column c of output plane p - R + k
+  // while plane p is applied.
+  T acc[K][S3S_ROWS][CE];
 #pragma unroll
   for (int k = 0; k < K; ++k)
 #pragma unroll
-    for (int r = 0; r < S3S_ROWS; ++r) acc[k][r] = Prim<ACC_ADD, T>::id();
-  const int64_t ps = z0 - R, pend = z1 - 1 + R;  // planes ps .. pend
+    for (int r = 0; r < S3S_ROWS; ++r)
+#pragma unroll
+      for (int c = 0; c < CE; ++c) acc[k][r][c] = Prim<ACC_ADD, T>::id();
+  const int ps = (int)z0 - R, pend = (int)z1 - 1 + R;  // planes ps .. pend
 #pragma unroll
   for (int i = 0; i < S3S_STAGES - 1; ++i) {
     if (ps + i <= pend) issue(ps + i, i);
     cp_async_commit();
   }
-  const int64_t gx = x0 + tx;
+  const int64_t gx = x0 + tx * CE;
   const int64_t gyt = y0 + ty * S3S_ROWS;
+  T *o = static_cast<T *>(a.out) + z0 * hw + gyt * a.w + gx;
+  // rows of this thread inside the array; columns likewise
+  const int nrow = gyt + S3S_ROWS <= a.h ? S3S_ROWS : (int)(a.h - gyt > 0 ? a.h - gyt : 0);
+  const int ncol = gx + CE <= a.w ? CE : (int)(a.w - gx > 0 ? a.w - gx : 0);
+  const bool whole = (CE == 1 || vec) && ncol == CE && nrow == S3S_ROWS;  // every output, 8-byte stores
   T wr[K * K * K];  // the weights, in registers (read once from the parameter)
 #pragma unroll
   for (int t = 0; t < K * K * K; ++t) wr[t] = W.w[t];
   int buf = 0;
-  auto step = [&](int64_t p, auto rot) {
-    constexpr int ROT = decltype(rot)::value;
+#pragma unroll 3
+  for (int p = ps; p <= pend; ++p) {
     cp_async_wait<S3S_STAGES - 2>();  // plane p's copies (this thread's) have landed
     __syncthreads();                  // ... and every thread's; the buffer of plane p-1 is free
-    {
-      const int64_t pn = p + S3S_STAGES - 1;
-      const int nb = buf == 0 ? S3S_STAGES - 1 : buf - 1;
-      if (pn <= pend) issue(pn, nb);
-      cp_async_commit();
-    }
+    if (p + S3S_STAGES - 1 <= pend) issue(p + S3S_STAGES - 1, buf == 0 ? S3S_STAGES - 1 : buf - 1);
+    cp_async_commit();
     // plane p: weight plane (p - z) + R for output z = p - R + k is 2R - k
-    const T *src = &plane[buf][ty * S3S_ROWS][tx + PX - R];
+    const T *srcp = &plane[buf][ty * S3S_ROWS][tx * CE + PX];
 #pragma unroll
     for (int ir = 0; ir < S3S_ROWS + 2 * R; ++ir) {
-      T xv[K];
+      T xv[CE + 2 * R];  // columns -1 .. CE of this thread's first column
+      if constexpr (CE == 2) {
+        const uint64_t q = *reinterpret_cast<const uint64_t *>(srcp + ir * PW);
+        memcpy(&xv[1], &q, 8);
+      } else {
 #pragma unroll
-      for (int dx = 0; dx < K; ++dx) xv[dx] = src[ir * PW + dx];
+        for (int c = 0; c < CE; ++c) xv[1 + c] = srcp[ir * PW + c];
+      }
+      xv[0] = srcp[ir * PW - 1];
+      xv[CE + 1] = srcp[ir * PW + CE];
 #pragma unroll
       for (int dyi = 0; dyi < K; ++dyi) {
         const int r = ir - dyi;
@@ -260,32 +309,44 @@ stencil3d_stream_kernel(const __grid_constant__ Stencil3Args a, const __grid_con
           for (int dx = 0; dx < K; ++dx) {
             const int t = ((2 * R - k) * K + dyi) * K + dx;
             if (!s3_tap<PAT>(t, mask)) continue;
-            T &ac = acc[(k + ROT) % K][r];
-            ac = fma_tap(wr[t], xv[dx], ac);
+#pragma unroll
+            for (int c = 0; c < CE; ++c) acc[k][r][c] = fma_tap(wr[t], xv[c + dx], acc[k][r][c]);
           }
         }
       }
     }
     // output plane p - R is complete
-    constexpr int S0 = ROT % K;
-    const int64_t zo = p - R;
-    if (zo >= z0 && gx < a.w) {
-      T *o = out + zo * hw + gyt * a.w + gx;
+    if (p - R >= (int)z0) {
+      if (whole) {
+        T *w = o;
 #pragma unroll
-      for (int r = 0; r < S3S_ROWS; ++r)
-        if (gyt + r < a.h) o[r * a.w] = acc[S0][r];
+        for (int r = 0; r < S3S_ROWS; ++r, w += a.w) {
+          if constexpr (CE == 2) {
+            uint64_t q;
+            memcpy(&q, acc[0][r], 8);
+            __stcs(reinterpret_cast<unsigned long long *>(w), (unsigned long long)q);
+          } else {
+            __stcs(w, acc[0][r][0]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < S3S_ROWS; ++r)
+#pragma unroll
+          for (int c = 0; c < CE; ++c)
+            if (r < nrow && c < ncol) o[r * a.w + c] = acc[0][r][c];
+      }
+      o += hw;
     }
 #pragma unroll
-    for (int r = 0; r < S3S_ROWS; ++r) acc[S0][r] = Prim<ACC_ADD, T>::id();
+    for (int r = 0; r < S3S_ROWS; ++r)
+#pragma unroll
+      for (int c = 0; c < CE; ++c) {
+        acc[0][r][c] = acc[1][r][c];
+        acc[1][r][c] = acc[2][r][c];
+        acc[2][r][c] = Prim<ACC_ADD, T>::id();
+      }
     buf = buf == S3S_STAGES - 1 ? 0 : buf + 1;
-  };
-  for (int64_t p = ps;;) {
-    step(p, std::integral_constant<int, 0>());
-    if (++p > pend) break;
-    step(p, std::integral_constant<int, 1>());
-    if (++p > pend) break;
-    step(p, std::integral_constant<int, 2>());
-    if (++p > pend) break;
   }
   cp_async_wait<0>();  // no copy outlives the CTA (the trailing groups are empty)
 }
@@ -317,8 +378,8 @@ int stencil3d_typed(const Stencil3Args &a, const void *weights, cudaStream_t s) 
   if (a.rz == 1 && a.ry == 1 && a.rx == 1) {
     // 3x3x3: the plane-streaming kernel, its tap pattern fixed at compile time
     // where it is dense or the 7-point star.
-    const int64_t sx = cdiv_h(a.w, S3S_TX), sy = cdiv_h(a.h, S3S_OY);
-    if (sx <= 0x7fffffffll && sy <= 65535) {
+    const int64_t sx = cdiv_h(a.w, S3S_TX * s3_cols<T>()), sy = cdiv_h(a.h, S3S_OY);
+    if (sx <= 0x7fffffffll && sy <= 65535 && a.d <= 0x7ffffff0ll) {
       uint32_t mask = 0;
       for (int t = 0; t < 27; ++t)
         if (!(W.w[t] == T(0))) mask |= 1u << t;
@@ -327,9 +388,13 @@ int stencil3d_typed(const Stencil3Args &a, const void *weights, cudaStream_t s) 
       const void *fn = pat == 0 ? (const void *)stencil3d_stream_kernel<T, 0>
                        : pat == 1 ? (const void *)stencil3d_stream_kernel<T, 1>
                                   : (const void *)stencil3d_stream_kernel<T, 2>;
-      int per_sm = 0;
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, S3S_THREADS, 0) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
+      static std::atomic<int> resident_ctas[3];
+      int per_sm = resident_ctas[pat].load(std::memory_order_relaxed);
+      if (per_sm == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, S3S_THREADS, 0) != cudaSuccess || per_sm < 1)
+          per_sm = 1;
+        resident_ctas[pat].store(per_sm, std::memory_order_relaxed);
+      }
       const int64_t zchunk = s3_zchunk(sx * sy, a.d, (int64_t)device_info().sms * per_sm);
       const int64_t nz = cdiv_h(a.d, zchunk);
       const int vec = (reinterpret_cast<uintptr_t>(a.in) % 16 == 0) && ((a.w * (int64_t)sizeof(T)) % 16 == 0);
