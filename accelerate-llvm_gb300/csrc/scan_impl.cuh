@@ -964,7 +964,7 @@ scan_zip_tma_kernel(const __grid_constant__ CUtensorMap tin, const __grid_consta
 }
 
 // --------------------------------------------------------------------------
-// Row scans (rank >= 2): one CTA per row, chunks of 256 x 4 elements with a
+// Row scans (rank >= 2, and short 1-D arrays): one CTA per row, in chunks with a
 // carried prefix.  in/out rows have pitches in_pitch / out_pitch (elements).
 struct RowScanArgs {
   const void *in;
@@ -983,88 +983,122 @@ struct RowScanArgs {
   uint64_t mapc;     // MAP kernels: the constant c (bits of one element)
 };
 
+// A CTA takes a row in chunks of blockDim x K elements (a row of up to 16,384
+// 32-bit elements is one chunk); a warp owns 32 K consecutive ones.  A chunk's
+// loads are coalesced and all in flight at once, the next chunk's (or row's)
+// before this one is worked on; the warp turns them in shared memory into K
+// consecutive elements per thread (rows of an odd pitch, free of bank
+// conflicts), scans those, and turns them back for coalesced stores, so the
+// only barrier of a chunk is the one that makes the warps' totals known.  The
+// carried prefix is kept by every thread.
+// Bound: a short row by the latency of its one chunk, many rows by issue.
+// Measured on a GB300 against chunks of 1024 elements, loaded one at a time
+// with three barriers each:
+// 1001 x 4099 Float32, compensated, 16.6 -> 9.6 us; 600 x 8000 16.2 -> 10.4; 64
+// x 64,000 59 -> 17; 3000 x 100 Float64 42 -> 7.8.
+constexpr int ROWS_MAXT = 1024;
+template <class T> constexpr int rows_k() { return sizeof(T) == 4 ? 16 : 8; }
+// 1-D arrays of at most one chunk take this kernel too, with one CTA: no tensor
+// maps, ticket or look-back.  10,007 elements: Int32 5.8 -> 3.3 us, Float32 7.5
+// -> 3.8; at one chunk (16,384) 4.9 -> 4.7 and 6.1 -> 5.4, at two chunks the
+// tile kernel is faster (20,000 Int32: 7.0 against 6.9).
+template <class T> constexpr int64_t rows_1d() { return ROWS_MAXT * rows_k<T>(); }
+
 template <int OP, class T, int PREC, bool R2L, bool ZIP = false, bool MAP = false>
-__global__ void __launch_bounds__(256) scan_rows_kernel(RowScanArgs a) {
+__global__ void __launch_bounds__(ROWS_MAXT, 1) scan_rows_kernel(RowScanArgs a) {
   using A = Acc<OP, T, PREC>;
   using S = typename A::S;
-  constexpr int K = 4;
-  constexpr int CH = 256 * K;
-  __shared__ S s_warp[8];
-  __shared__ S s_carry;
+  constexpr int K = rows_k<T>(), PITCH = K + 1, RPI = 32 / K;  // RPI: thread rows per 32 elements
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ S s_warp[2][ROWS_MAXT / 32];
+  const int nt = blockDim.x, nw = nt >> 5;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  T *wbuf = reinterpret_cast<T *>(smem_raw) + warp * (32 * PITCH);
+  T *turn = wbuf + (lane / K) * PITCH + lane % K;  // element j * 32 + lane of the warp: turn[j * RPI * PITCH]
+  T *row = wbuf + lane * PITCH;                    // element lane * K + j: row[j]
   const T idT = Prim<OP, T>::id();
-  for (int64_t r = blockIdx.x; r < a.outer; r += gridDim.x) {
-    const T *src = static_cast<const T *>(a.in) + r * a.in_pitch;
-    const T *src2 = ZIP ? static_cast<const T *>(a.in2) + r * a.in_pitch : nullptr;
+  const T mapc = from_bits<T>(a.mapc);
+  (void)mapc;
+  const int64_t ch = (int64_t)nt * K;
+  const int64_t nch = (a.inner + ch - 1) / ch;
+  // elements 0 * 32 + lane, 1 * 32 + lane, ... of this warp's part of chunk c of row r
+  auto load = [&](int64_t r, int64_t c, T (&x)[K]) {
+    const int64_t e0 = c * ch + warp * (32 * K) + lane;
+    const T *src = static_cast<const T *>(a.in) + r * a.in_pitch + e0;
+    const T *src2 = ZIP ? static_cast<const T *>(a.in2) + r * a.in_pitch + e0 : nullptr;
     (void)src2;
+    const int64_t left = a.inner - e0;  // elements of the row from e0 on
+    auto elem = [&](int j) -> T {
+      if constexpr (ZIP) return zip_elem(a.zop, src[j * 32], src2[j * 32]);
+      else if constexpr (MAP) return zip_elem(a.zop, src[j * 32], mapc);
+      else return src[j * 32];
+    };
+    if (left > 32 * (K - 1)) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) x[j] = elem(j);
+    } else {
+#pragma unroll
+      for (int j = 0; j < K; ++j) x[j] = j * 32 < left ? elem(j) : idT;
+    }
+  };
+  T next[K];
+  if ((int64_t)blockIdx.x < a.outer) load(blockIdx.x, R2L ? nch - 1 : 0, next);
+  int par = 0;
+  for (int64_t r = blockIdx.x; r < a.outer; r += gridDim.x) {
     T *dst = static_cast<T *>(a.out) + r * a.out_pitch;
-    if (tid == 0) s_carry = a.has_seed ? A::lift(from_bits<T>(a.seed)) : A::id();
-    __syncthreads();
-    const int64_t nch = (a.inner + CH - 1) / CH;
-    for (int64_t ci = 0; ci < nch; ++ci) {
+    S carry = a.has_seed ? A::lift(from_bits<T>(a.seed)) : A::id();
+    for (int64_t ci = 0; ci < nch; ++ci, par ^= 1) {
       const int64_t c = R2L ? nch - 1 - ci : ci;
-      const int64_t e0 = c * CH + (int64_t)tid * K;
-      T x[K];
 #pragma unroll
-      for (int j = 0; j < K; ++j) {
-        x[j] = idT;
-        if (e0 + j < a.inner) {
-          if constexpr (ZIP) x[j] = zip_elem(a.zop, src[e0 + j], src2[e0 + j]);
-          else if constexpr (MAP) x[j] = zip_elem(a.zop, src[e0 + j], from_bits<T>(a.mapc));
-          else x[j] = src[e0 + j];
-        }
-      }
-      S agg;
-      if (!R2L) { agg = A::lift(x[0]); for (int j = 1; j < K; ++j) agg = A::push(agg, x[j]); }
-      else { agg = A::lift(x[K - 1]); for (int j = K - 2; j >= 0; --j) agg = A::push(agg, x[j]); }
-      S incl, ex;
-      if (!R2L) {
-        incl = warp_scan_incl<A>(agg);
-        S up = shfl_up(incl, 1);
-        ex = lane == 0 ? A::id() : up;
-        if (lane == 31) s_warp[warp] = incl;
-      } else {
-        incl = warp_scan_incl_rev<A>(agg);
-        S dn = shfl_down(incl, 1);
-        ex = lane == 31 ? A::id() : dn;
-        if (lane == 0) s_warp[warp] = incl;
-      }
+      for (int j = 0; j < K; ++j) turn[j * RPI * PITCH] = next[j];
+      __syncwarp();
+      if (ci + 1 < nch) load(r, R2L ? c - 1 : c + 1, next);
+      else if (r + gridDim.x < a.outer) load(r + gridDim.x, R2L ? nch - 1 : 0, next);
+      S agg = A::lift(row[R2L ? K - 1 : 0]);
+#pragma unroll
+      for (int j = 1; j < K; ++j) agg = A::push(agg, row[R2L ? K - 1 - j : j]);
+      const S incl = R2L ? warp_scan_incl_rev<A>(agg) : warp_scan_incl<A>(agg);
+      S ex = R2L ? shfl_down(incl, 1) : shfl_up(incl, 1);
+      if (lane == (R2L ? 31 : 0)) ex = A::id();
+      if (lane == (R2L ? 0 : 31)) s_warp[par][warp] = incl;
       __syncthreads();
-      S wpre = A::id();
-      if (!R2L) { for (int w = 0; w < warp; ++w) wpre = A::comb(wpre, s_warp[w]); }
-      else { for (int w = warp + 1; w < 8; ++w) wpre = A::comb(wpre, s_warp[w]); }
-      S bagg = s_warp[0];
-      for (int w = 1; w < 8; ++w) bagg = A::comb(bagg, s_warp[w]);
-      const S carry = s_carry;
+      // the chunk's total, and that of the warps before (R2L: after) this one
+      const S wv = lane < nw ? s_warp[par][lane] : A::id();
+      const S ws = R2L ? warp_scan_incl_rev<A>(wv) : warp_scan_incl<A>(wv);
+      const S total = shfl_idx(ws, R2L ? 0 : 31);
+      S wpre = shfl_idx(ws, (R2L ? warp + 1 : warp - 1) & 31);
+      if (warp == (R2L ? nw - 1 : 0)) wpre = A::id();
       S run = R2L ? A::comb(A::comb(ex, wpre), carry) : A::comb(carry, A::comb(wpre, ex));
-      if (!R2L) {
 #pragma unroll
-        for (int j = 0; j < K; ++j) {
-          T yv;
-          if (a.exclusive) { yv = A::lower(run); run = A::push(run, x[j]); }
-          else { run = A::push(run, x[j]); yv = A::lower(run); }
-          if (e0 + j < a.inner) dst[e0 + j] = yv;
-        }
+      for (int jj = 0; jj < K; ++jj) {
+        const int j = R2L ? K - 1 - jj : jj;
+        const T x = row[j];
+        T y;
+        if (a.exclusive) { y = A::lower(run); run = A::push(run, x); }
+        else { run = A::push(run, x); y = A::lower(run); }
+        row[j] = y;
+      }
+      carry = R2L ? A::comb(total, carry) : A::comb(carry, total);
+      __syncwarp();
+      const int64_t e0 = c * ch + warp * (32 * K) + lane;
+      const int64_t left = a.inner - e0;
+      T *to = dst + e0;
+      if (left > 32 * (K - 1)) {
+#pragma unroll
+        for (int j = 0; j < K; ++j) to[j * 32] = turn[j * RPI * PITCH];
       } else {
 #pragma unroll
-        for (int j = K - 1; j >= 0; --j) {
-          T yv;
-          if (a.exclusive) { yv = A::lower(run); run = A::push(run, x[j]); }
-          else { run = A::push(run, x[j]); yv = A::lower(run); }
-          if (e0 + j < a.inner) dst[e0 + j] = yv;
-        }
+        for (int j = 0; j < K; ++j)
+          if (j * 32 < left) to[j * 32] = turn[j * RPI * PITCH];
       }
-      __syncthreads();
-      if (tid == 0) s_carry = R2L ? A::comb(bagg, carry) : A::comb(carry, bagg);
-      __syncthreads();
+      __syncwarp();
     }
     if (tid == 0) {
-      const T total = A::lower(s_carry);
+      const T total = A::lower(carry);
       if (a.sums) static_cast<T *>(a.sums)[r] = total;
       if (a.total_at_end) dst[a.inner] = total;
       if (a.seed_at_end) dst[a.inner] = from_bits<T>(a.seed);
     }
-    __syncthreads();
   }
 }
 
@@ -1145,10 +1179,14 @@ int launch_scan_l2(Workspace *w, const T *in, T *out, T *total_out, T *seed_out,
   auto kern = scan_l2_kernel<OP, T, PREC, R2L, PROD, SEG>;
   static std::atomic<uint64_t> attr_done{0};
   smem_attrs_once(kern, (int)smem, attr_done);
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, L2S_THREADS, smem) != cudaSuccess || per_sm < 1) {
-    cudaGetLastError();
-    return ACC_OK;
+  static std::atomic<int> resident{0};  // CTAs per SM, asked for once
+  int per_sm = resident.load(std::memory_order_relaxed);
+  if (per_sm == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, L2S_THREADS, smem) != cudaSuccess || per_sm < 1) {
+      cudaGetLastError();
+      return ACC_OK;
+    }
+    resident.store(per_sm, std::memory_order_relaxed);
   }
   int st = ws_status(w, (size_t)ntiles * 2);
   if (st) return st;
@@ -1188,33 +1226,6 @@ int launch_scan_l2(Workspace *w, const T *in, T *out, T *total_out, T *seed_out,
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tin, tout, a, tin2);
   *launched = true;
   return cuda_status(e);
-}
-
-// Large arrays take the persistent kernel (over a fused map as well).  The
-// tile kernel's size below that: 2 sub-tiles (64 KiB, 3 CTAs per SM) by
-// default, the faster of the two on GB300 at 2^25..2^28 elements;
-// ACC_GB300_SCAN_SUB=1 selects 32 KiB tiles (6 CTAs per SM).  A scan over a
-// fused map (MAP: map (\x -> mop x c)) always takes the 64 KiB tiles there.
-template <int OP, class T, int PREC, bool R2L, bool MAP = false>
-int launch_scan_1d(Workspace *w, const T *in, T *out, T *total_out, T *seed_out, int64_t n,
-                   bool has_seed, bool exclusive, uint64_t seed, cudaStream_t s, int mop = 0,
-                   uint64_t mapc = 0) {
-  // Arrays of at least four 32 KiB tiles per SM take the persistent
-  // L2-re-read kernel (ACC_GB300_SCAN_KERNEL=tile keeps the tile kernel).
-  static const bool l2k = !(getenv("ACC_GB300_SCAN_KERNEL") && strcmp(getenv("ACC_GB300_SCAN_KERNEL"), "tile") == 0);
-  if (l2k && n * (int64_t)sizeof(T) >= (int64_t)device_info().sms * 4 * L2S_TILE) {
-    bool launched = false;
-    const int st = launch_scan_l2<OP, T, PREC, R2L, MAP ? 1 : 0>(w, in, out, total_out, seed_out, n, has_seed,
-                                                                 exclusive, seed, s, &launched, nullptr, mop, mapc);
-    if (st || launched) return st;
-  }
-  if constexpr (MAP)
-    return launch_scan_1d_sub<OP, T, PREC, R2L, 2, true>(w, in, out, total_out, seed_out, n, has_seed, exclusive,
-                                                          seed, s, mop, mapc);
-  static const int sub = getenv("ACC_GB300_SCAN_SUB") ? atoi(getenv("ACC_GB300_SCAN_SUB")) : 2;
-  if (sub == 2)
-    return launch_scan_1d_sub<OP, T, PREC, R2L, 2>(w, in, out, total_out, seed_out, n, has_seed, exclusive, seed, s);
-  return launch_scan_1d_sub<OP, T, PREC, R2L, 1>(w, in, out, total_out, seed_out, n, has_seed, exclusive, seed, s);
 }
 
 // Short rows, many of them: one warp per row.  The warp walks the row in
@@ -1283,10 +1294,57 @@ int launch_scan_rows(const RowScanArgs &a, cudaStream_t s) {
     scan_rows_warp_kernel<OP, T, PREC, R2L, ZIP, MAP><<<(unsigned)blocks, 256, 0, s>>>(a);
     return check_launch();
   }
+  // as many threads as a row needs, at ROWS_K elements each
+  constexpr int K = rows_k<T>();
+  int64_t nt = cdiv_h(cdiv_h(a.inner, K), 32) * 32;
+  if (nt > ROWS_MAXT) nt = ROWS_MAXT;
+  int64_t per_sm = 2048 / nt;
+  if (per_sm > 16) per_sm = 16;
   int64_t blocks = a.outer;
-  if (blocks > (int64_t)d.sms * 8) blocks = (int64_t)d.sms * 8;
-  scan_rows_kernel<OP, T, PREC, R2L, ZIP, MAP><<<(unsigned)blocks, 256, 0, s>>>(a);
+  if (blocks > (int64_t)d.sms * per_sm) blocks = (int64_t)d.sms * per_sm;
+  const size_t smem = (size_t)nt * (K + 1) * sizeof(T);
+  auto kern = scan_rows_kernel<OP, T, PREC, R2L, ZIP, MAP>;
+  static std::atomic<uint64_t> attr_done{0};
+  smem_attrs_once(kern, ROWS_MAXT * (K + 1) * (int)sizeof(T), attr_done, false);
+  kern<<<(unsigned)blocks, (unsigned)nt, smem, s>>>(a);
   return check_launch();
+}
+
+// Short arrays take the row kernel, large ones the persistent kernel (over a
+// fused map as well).  The
+// tile kernel's size below that: 2 sub-tiles (64 KiB, 3 CTAs per SM) by
+// default, the faster of the two on GB300 at 2^25..2^28 elements;
+// ACC_GB300_SCAN_SUB=1 selects 32 KiB tiles (6 CTAs per SM).  A scan over a
+// fused map (MAP: map (\x -> mop x c)) always takes the 64 KiB tiles there.
+template <int OP, class T, int PREC, bool R2L, bool MAP = false>
+int launch_scan_1d(Workspace *w, const T *in, T *out, T *total_out, T *seed_out, int64_t n,
+                   bool has_seed, bool exclusive, uint64_t seed, cudaStream_t s, int mop = 0,
+                   uint64_t mapc = 0) {
+  // Arrays of at least four 32 KiB tiles per SM take the persistent
+  // L2-re-read kernel (ACC_GB300_SCAN_KERNEL=tile keeps the tile kernel).
+  if (n <= rows_1d<T>()) {
+    RowScanArgs a{};
+    a.in = in; a.out = out; a.sums = total_out;
+    a.outer = 1; a.inner = n; a.in_pitch = n; a.out_pitch = n;
+    a.seed = seed; a.has_seed = has_seed; a.exclusive = exclusive;
+    a.seed_at_end = seed_out != nullptr;  // always out + n
+    a.zop = mop; a.mapc = mapc;
+    return launch_scan_rows<OP, T, PREC, R2L, false, MAP>(a, s);
+  }
+  static const bool l2k = !(getenv("ACC_GB300_SCAN_KERNEL") && strcmp(getenv("ACC_GB300_SCAN_KERNEL"), "tile") == 0);
+  if (l2k && n * (int64_t)sizeof(T) >= (int64_t)device_info().sms * 4 * L2S_TILE) {
+    bool launched = false;
+    const int st = launch_scan_l2<OP, T, PREC, R2L, MAP ? 1 : 0>(w, in, out, total_out, seed_out, n, has_seed,
+                                                                 exclusive, seed, s, &launched, nullptr, mop, mapc);
+    if (st || launched) return st;
+  }
+  if constexpr (MAP)
+    return launch_scan_1d_sub<OP, T, PREC, R2L, 2, true>(w, in, out, total_out, seed_out, n, has_seed, exclusive,
+                                                          seed, s, mop, mapc);
+  static const int sub = getenv("ACC_GB300_SCAN_SUB") ? atoi(getenv("ACC_GB300_SCAN_SUB")) : 2;
+  if (sub == 2)
+    return launch_scan_1d_sub<OP, T, PREC, R2L, 2>(w, in, out, total_out, seed_out, n, has_seed, exclusive, seed, s);
+  return launch_scan_1d_sub<OP, T, PREC, R2L, 1>(w, in, out, total_out, seed_out, n, has_seed, exclusive, seed, s);
 }
 
 // A 1-D scan over zipWith g in in2 (g = zop): the zipped tile kernel when
