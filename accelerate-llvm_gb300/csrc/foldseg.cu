@@ -244,16 +244,24 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 //     first boundary and after its last one are carried out;
 //   * a segmented CTA scan ((f1,v1).(f2,v2) = (f1|f2, f2 ? v2 : v1 `f` v2))
 //     gives every row the value carried in from earlier rows of the tile, and
-//     the tile's own carried-out value, which is final at once: the tile
-//     publishes it (flag 2 when the tile holds a boundary, 1 when it lies
-//     inside one segment) before it looks back;
+//     the tile's own carried-out value (flag 2 when the tile holds a boundary,
+//     1 when it lies inside one segment);
 //   * the parked results are written out in one coalesced pass, except the
-//     segment that closes at the tile's first boundary, which needs the
-//     value carried in from earlier tiles: a decoupled look-back that stops
-//     at the nearest tile holding a boundary (usually the previous one).
-// An extra tile past the last value closes the segments that end at the
-// very end of the row.  Two launches: the index pre-pass and the tile pass.  Offsets that decrease or leave [0, n] raise
-// ACC_ERR_INDEX; the tile then writes nothing but still publishes.
+//     segment that closes at the tile's first boundary, which also needs the
+//     values carried in from earlier tiles: its part goes to the tile's slot
+//     with the carried-out value, and foldseg_fix completes those segments from
+//     the slots, each from the nearest earlier tile that holds a boundary
+//     (usually the previous one).
+// An extra tile past the last value closes the segments that end at the very
+// end of the row.  Three launches: the index pre-pass, the tiles and the
+// completion; one for short calls.  Offsets that decrease or leave [0, n] raise
+// ACC_ERR_INDEX; the tile then writes nothing.
+// Bound: issue (about 38 thread instructions per value, compensated).  A tile
+// that completed its first segment itself, by a decoupled look-back, held its
+// shared memory for 7,400 cycles of polls and 2,100 of drawing a ticket, of
+// 19,800 (2^22 values); the tiles now wait for no one.  2^26 Float32 values in
+// 2^20 lognormal segments, compensated: 115 -> 100 us, plain 88 -> 75, Int32 max
+// 88 -> 76 (the index pre-pass is 7 of them).
 constexpr int FT_THREADS = 256;
 constexpr int FT_ROW_BYTES = 128;
 constexpr int FT_CAP = 512;   // tile-relative offsets (and their results) held in shared memory
@@ -270,14 +278,34 @@ struct SegTileArgs {
   int64_t full_rows, ntiles;
   uint64_t seed;
   int has_seed;
-  const uint64_t *tidx;  // per tile: epoch tag << 35 | first offset index >= the tile start
-  uint64_t *status;
-  uint32_t *ticket;
+  struct SegSlot *slots;  // per tile
+  const uint64_t *tidx;  // per tile: epoch tag << 35 | first offset index >= the tile start; small: unused
+  int small;             // 1: the CTA keeps all the offsets in shared memory; 2: and scans them from the lengths
+  uint32_t *done;  // small: tiles finished (zero between calls)
   uint32_t *err;
   uint32_t epoch;
 };
 
+// What a tile leaves for the segments that cross its edges.
+struct __align__(16) SegSlot {
+  uint64_t carry;    // state carried out to the right (bits)
+  uint64_t first;    // state of the part before the tile's first boundary
+  int64_t first_id;  // the segment that closes there, or -1
+  int64_t boundary;  // 1: the tile holds a boundary, so its carry starts inside it
+};
+
 constexpr int TIDX_SHIFT = 35;  // offset indices below 2^35; the epoch above
+
+// Short calls (at most FT_SMALL segments, at most two tiles per SM) take one
+// launch: each CTA reads all the offsets (or the lengths, which it scans) into
+// shared memory and finds its tile's first and last offset by counting.
+// 100,003 Int32 values in 1,562 segments by lengths, device time: 23.4 us in
+// three launches (scan of the lengths, index, tiles) -> 13.5; by offsets 17.1
+// -> 13.4.  At the limits, 10^6 Float32 values: 4,000 segments by offsets 14.8 ->
+// 13.8 us, 15,625 segments (three launches) 15.0 -> 13.1.
+constexpr int FT_SMALL = 4096;
+constexpr int FT_PER = (FT_SMALL + FT_THREADS) / FT_THREADS;  // most offsets per thread
+static_assert(FT_PER % 2 == 1 && FT_PER * FT_THREADS >= FT_SMALL + 1, "an odd number (free of bank conflicts) holds them all");
 
 // Pre-pass: tidx[t] = the first k with off[k] >= t * te (t < ntiles), and
 // tidx[ntiles] = nseg + 1, each tagged with the call's epoch so that no
@@ -307,25 +335,60 @@ __global__ void foldseg_tile_index(const OT *off, int64_t nseg, int64_t ntiles, 
   }
 }
 
-// Look-back slot of the tiled foldSeg: tag = epoch << 3 | flag.
-template <class S>
-__device__ __forceinline__ void publish_seg(uint64_t *status, int64_t t, uint32_t epoch, uint32_t flag, S v) {
-  uint64_t b = to_bits(v);
-  uint64_t tag = (uint64_t)((epoch << 3) | flag) << 32;
-  if constexpr (sizeof(S) == 8) st_relaxed_u64(status + 2 * t + 1, tag | (b >> 32));
-  st_relaxed_u64(status + 2 * t, tag | (b & 0xffffffffull));
-}
-template <class S>
-__device__ __forceinline__ uint32_t decode_seg(SlotWords s, uint32_t epoch, S &v) {
-  const uint32_t tag = (uint32_t)(s.w0 >> 32);
-  if ((tag >> 3) != epoch) return 0;
-  uint64_t b = s.w0 & 0xffffffffull;
-  if constexpr (sizeof(S) == 8) {
-    if ((uint32_t)(s.w1 >> 32) != tag) return 0;
-    b |= (s.w1 & 0xffffffffull) << 32;
+// Complete the segment that closes at the first boundary of tile t0 + lane, for
+// 32 tiles (warp-collective): the carried-out values of the tiles since the
+// nearest earlier boundary, then the tile's own first part.  The previous tile
+// usually holds that boundary; where it does not, the warp walks back together,
+// 32 slots at a time.
+template <int OP, class T, int PREC>
+__device__ __forceinline__ void seg_complete(const SegTileArgs &a, int64_t t0) {
+  using A = Acc<OP, T, PREC>;
+  using S = typename A::S;
+  const int lane = threadIdx.x & 31;
+  const int64_t t = t0 + lane;
+  auto word = [&](const void *p) { return ld_relaxed_u64(static_cast<const uint64_t *>(p)); };
+  int64_t id = -1;
+  S carry = A::id();
+  bool closed = true;
+  if (t < a.ntiles) {
+    const SegSlot *prev = a.slots + (t > 0 ? t - 1 : 0);
+    id = (int64_t)word(&a.slots[t].first_id);
+    const uint64_t pc = word(&prev->carry), pb = word(&prev->boundary);
+    if (id >= 0 && id < a.nseg && t > 0) {
+      carry = from_bits<S>(pc);
+      closed = pb != 0;
+    }
   }
-  v = from_bits<S>(b);
-  return tag & 3u;
+  unsigned open = __ballot_sync(0xffffffffu, !closed);
+  while (open) {
+    const int l = __ffs(open) - 1;
+    open &= open - 1;
+    S acc = shfl_idx(carry, l);
+    for (int64_t k = t0 + l - 2;; k -= 32) {
+      const int64_t q = k - lane;
+      S v = A::id();
+      bool stop = q < 0;
+      if (!stop) {
+        v = from_bits<S>(word(&a.slots[q].carry));
+        stop = word(&a.slots[q].boundary) != 0;
+      }
+      const unsigned sm = __ballot_sync(0xffffffffu, stop);
+      const int ks = sm ? __ffs(sm) - 1 : 32;
+      if (lane > ks) v = A::id();
+      const S w = shfl_idx(warp_reduce_rev<A>(v), 0);
+      acc = A::comb(w, acc);
+      if (sm) break;
+    }
+    if (lane == l) carry = acc;
+  }
+  if (t < a.ntiles && id >= 0 && id < a.nseg) {
+    const S v = A::comb(carry, from_bits<S>(word(&a.slots[t].first)));
+    static_cast<T *>(a.out)[id] = A::lower(a.has_seed ? A::comb(A::lift(from_bits<T>(a.seed)), v) : v);
+  }
+}
+template <int OP, class T, int PREC>
+__global__ void __launch_bounds__(256) foldseg_fix(SegTileArgs a) {
+  seg_complete<OP, T, PREC>(a, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll);
 }
 
 template <int OP, class T, int PREC, class OT>
@@ -344,7 +407,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char *buf = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t bar;
-  __shared__ int64_t s_tile, s_kf, s_cnt, s_lo, s_hi, s_first_id;
+  __shared__ int64_t s_kf, s_cnt, s_lo, s_hi, s_first_id;
   __shared__ int s_offs[FT_CAP];
   __shared__ int s_rowh[FT_THREADS];  // per thread: first offset entry at or after its first value
   __shared__ S s_res[FT_CAP];         // per entry (or, in a slot tile, per boundary): a closed segment's state
@@ -354,33 +417,77 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
   __shared__ uint64_t s_bm[FT_THREADS];  // slot tiles: each thread's boundary positions
   __shared__ int s_base[FT_THREADS];     // slot tiles: each thread's first boundary slot
   __shared__ int s_nbw[NWARP];
+  __shared__ unsigned s_count;           // small: offsets before the tile, and (high half) before its end
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const OT *off = static_cast<const OT *>(a.off);
+  const OT *off = static_cast<const OT *>(a.off);  // small: in shared memory, below
   T *out = static_cast<T *>(a.out);
   const T idT = Prim<OP, T>::id();
 
+  const int64_t tile = blockIdx.x;
   if (tid == 0) {
-    const uint32_t dyn = atomicAdd(a.ticket, 1u);
-    if ((int64_t)dyn == a.ntiles - 1) *a.ticket = 0u;
-    s_tile = dyn;
     s_has_first = 0;
     s_bad = 0;
+    s_count = 0;
     mbar_init(&bar, 1);
     fence_mbar_init();
     mbar_expect_tx(&bar, FT_RPT * SUB_BYTES);
 #pragma unroll
     for (int u = 0; u < FT_RPT; ++u)
-      tma_load_2d(buf + u * SUB_BYTES, &tin, 0, (int)(((int64_t)dyn * FT_RPT + u) * FT_THREADS), &bar);
+      tma_load_2d(buf + u * SUB_BYTES, &tin, 0, (int)((tile * FT_RPT + u) * FT_THREADS), &bar);
   }
   __syncthreads();
-  const int64_t tile = s_tile;
   const int64_t tb = tile * TE;
   const bool last_tile = tile == a.ntiles - 1;
+  if (a.small) {
+    const OT *given = off;
+    OT *all = reinterpret_cast<OT *>(buf + FT_RPT * SUB_BYTES);
+    const int no = (int)a.nseg + 1, ng = a.small == 2 ? no - 1 : no;
+    const int per = ((no + FT_THREADS - 1) / FT_THREADS) | 1;  // consecutive offsets per thread, an odd number
+    {
+      OT mine[FT_PER];
+#pragma unroll
+      for (int j = 0; j < FT_PER; ++j) {
+        mine[j] = OT(0);
+        if (j < per && tid + j * FT_THREADS < ng) mine[j] = given[tid + j * FT_THREADS];
+      }
+#pragma unroll
+      for (int j = 0; j < FT_PER; ++j)
+        if (j < per) all[tid + j * FT_THREADS] = mine[j];
+    }
+    __syncthreads();
+    OT *mine = all + tid * per;
+    if (a.small == 2) {
+      // exclusive scan of the lengths, wrapping as scanl (+) 0 does
+      using U = typename IntBits<OT>::U;
+      U sum = 0;
+      for (int j = 0; j < per; ++j) sum += (U)mine[j];
+      const U incl = warp_scan_incl<Acc<ACC_ADD, U, 0>>(sum);
+      U *s_sum = reinterpret_cast<U *>(all + FT_PER * FT_THREADS);
+      if (lane == 31) s_sum[warp] = incl;
+      __syncthreads();
+      U run = incl - sum;
+      for (int w2 = 0; w2 < warp; ++w2) run += s_sum[w2];
+      for (int j = 0; j < per; ++j) {
+        const U len = (U)mine[j];
+        mine[j] = (OT)run;
+        run += len;
+      }
+    }
+    unsigned before = 0;  // of this thread's offsets: before the tile | before its end << 16
+    for (int j = 0; j < per; ++j)
+      if (tid * per + j < no)
+        before += ((int64_t)mine[j] < tb ? 1u : 0u) + ((int64_t)mine[j] < tb + TE ? 0x10000u : 0u);
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) atomicAdd(&s_count, before);
+    off = all;
+    __syncthreads();
+  }
   if (tid < 32) {
     // The offsets inside [tb, te) are [kf, ks); the last tile takes every
     // remaining one (ks = nseg + 1).
     const uint64_t tag = (uint64_t)a.epoch << TIDX_SHIFT, mask = (1ull << TIDX_SHIFT) - 1;
-    const uint64_t e0 = a.tidx[tile], e1 = a.tidx[tile + 1];
+    const uint64_t e0 = a.small ? tag | (s_count & 0xffffu) : a.tidx[tile];
+    const uint64_t e1 = a.small ? tag | (last_tile ? (uint64_t)(a.nseg + 1) : (uint64_t)(s_count >> 16)) : a.tidx[tile + 1];
     const int64_t vstart = (int64_t)off[0], vend = (int64_t)off[a.nseg];
     if (lane == 0) {
       const int64_t kf = (int64_t)(e0 & mask), ks = (int64_t)(e1 & mask);
@@ -442,8 +549,43 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
     if (lane == 0) raise_error(a.err, DEV_ERR_TIMEOUT);
     landed = mbar_wait_sleep(&bar, 0);
   }
-  // A tile whose load never landed is neither read nor published.
-  if (__syncthreads_or(!landed)) return;
+  // The tile's slot; short calls: the last tile to get here completes the
+  // segments that cross tiles, for all of them.
+  auto finish = [&](uint64_t carry, uint64_t first, int64_t first_id, bool boundary) {
+    if (tid == 0) {
+      SegSlot sl{carry, first, first_id, boundary ? 1 : 0};
+      uint4 q[2];
+      memcpy(q, &sl, sizeof(sl));
+      reinterpret_cast<uint4 *>(a.slots + tile)[0] = q[0];
+      reinterpret_cast<uint4 *>(a.slots + tile)[1] = q[1];
+    }
+    if (!a.small) return;
+    if (tid == 0) {
+      __threadfence();
+      s_bad = atomicAdd(a.done, 1u) == (uint32_t)(a.ntiles - 1) ? 2 : 0;
+    }
+    __syncthreads();
+    if (s_bad != 2) return;
+    __threadfence();
+    if (tid == 0) *a.done = 0u;
+    for (int64_t t0 = warp * 32; t0 < a.ntiles; t0 += FT_THREADS) seg_complete<OP, T, PREC>(a, t0);
+  };
+  // A tile whose load never landed is not read.
+  if (__syncthreads_or(!landed)) {
+    finish(0, 0, -1, true);
+    return;
+  }
+  // The values after the last whole row (TMA left zeros there; the positions
+  // past the last value are masked below).
+  if (a.full_rows >= tile * (FT_RPT * FT_THREADS) && a.full_rows < (tile + 1) * (FT_RPT * FT_THREADS)) {
+    const int64_t gi = a.full_rows * ITEMS + tid;
+    if (tid < ITEMS && gi < a.n) {
+      const int r = (int)(a.full_rows - tile * (FT_RPT * FT_THREADS)), rr = r % FT_THREADS;
+      *reinterpret_cast<T *>(buf + (r / FT_THREADS) * SUB_BYTES + rr * FT_ROW_BYTES + (((tid / VEC) ^ (rr & 7)) << 4) +
+                             (tid % VEC) * sizeof(T)) = static_cast<const T *>(a.in)[gi];
+    }
+    __syncthreads();
+  }
   const bool ok = s_bad == 0;
   if (!ok && tid == 0) raise_error(a.err, DEV_ERR_INDEX);
   const int lo = (int)s_lo, hi = (int)s_hi;
@@ -536,19 +678,10 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
   auto load_chunk = [&](int c, T (&x)[VEC]) {
     const int r = FT_RPT * tid + c / (ITEMS / VEC);  // row within the tile
     const int cc = c % (ITEMS / VEC);                // 16-byte chunk within the row
-    if (tile * (FT_RPT * FT_THREADS) + r < a.full_rows) {
-      const int rr = r % FT_THREADS;
-      const uint4 v = *reinterpret_cast<const uint4 *>(buf + (r / FT_THREADS) * SUB_BYTES + rr * FT_ROW_BYTES +
-                                                       ((cc ^ (rr & 7)) << 4));
-      memcpy(x, &v, 16);
-    } else {
-      const T *src = static_cast<const T *>(a.in);
-#pragma unroll
-      for (int q = 0; q < VEC; ++q) {
-        const int64_t gi = tb + tb0 + c * VEC + q;
-        x[q] = gi < a.n ? src[gi] : idT;
-      }
-    }
+    const int rr = r % FT_THREADS;
+    const uint4 v = *reinterpret_cast<const uint4 *>(buf + (r / FT_THREADS) * SUB_BYTES + rr * FT_ROW_BYTES +
+                                                     ((cc ^ (rr & 7)) << 4));
+    memcpy(x, &v, 16);
   };
   // Fast walk: when this thread's offsets are in shared memory they become
   // a bit mask of boundary positions (bm) and the boundaries take entries
@@ -558,7 +691,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
   static_assert(W <= 64, "one 64-bit boundary mask per thread");
   int64_t h_end = tid + 1 < FT_THREADS ? (int64_t)s_rowh[tid + 1] : cnt;
   if (h_end < h || h_end > cnt) h_end = cnt;
-  bool fast = !masked && ok && h_end <= FT_CAP;
+  bool fast = ok && h_end <= FT_CAP;
   uint64_t bm = 0, dm = 0;
   if (fast) {
     for (int64_t e = h; e < h_end; ++e) {
@@ -586,13 +719,14 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
         const bool bnd = (cb >> q) & 1u;
         if (bnd) s_res[hh] = acc;
         if (bnd && ((cd >> q) & 1u)) {
-          const int pos = tb0 + c * VEC + q;
-          do { ++hh; } while (hh < h_end && s_offs[hh] == pos);
+          const int at = tb0 + c * VEC + q;
+          do { ++hh; } while (hh < h_end && s_offs[hh] == at);
         } else {
           hh += bnd ? 1 : 0;
         }
         acc = bnd ? A::id() : acc;
-        acc = A::push(acc, x[q]);
+        const int pos = tb0 + c * VEC + q;
+        acc = A::push(acc, pos >= lo && pos < hi ? x[q] : idT);
       }
     }
     started = hh != h0;
@@ -665,9 +799,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
   }
   __syncthreads();
 
-  // ---- publish; the parked results leave; look back for the segment closing
-  // at the tile's first boundary (entry 0)
-  if (tid == 0) publish_seg<S>(a.status, tile, a.epoch, s_tile_f ? 2u : 1u, s_tile_v);
+  // ---- the parked results leave
   if (ok) {
     const int64_t nres = cnt < FT_CAP ? cnt : FT_CAP;
     for (int64_t e = 1 + tid; e < nres; e += FT_THREADS)
@@ -682,73 +814,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
         out[kf + e - 1] = A::lower(a.has_seed ? A::comb(A::lift(z), v) : v);
       }
   }
-  if (warp == 0) {
-    if (s_has_first && s_first_id >= 0) {
-      constexpr int LB = 4;
-      S carry = A::id();
-      int64_t k0 = 0;
-      bool gave_up = false;
-      uint32_t it = 0;
-      uint64_t t_wait = 0;
-      while (true) {
-        uint32_t fl[LB];
-        S v[LB];
-#pragma unroll
-        for (int i = 0; i < LB; ++i) {
-          fl[i] = tile - 1 - (k0 + lane * LB + i) >= 0 ? 0u : 2u;
-          v[i] = A::id();
-        }
-        bool resolved = false, whole = false;
-        int kp = 32;
-        while (true) {
-          const int kp0 = lb_stop_lane<LB>(fl);
-          SlotWords sw[LB];
-#pragma unroll
-          for (int i = 0; i < LB; ++i) {
-            sw[i] = SlotWords{0ull, 0ull};
-            if (fl[i] == 0 && lane <= kp0) sw[i] = ld_slot(a.status + 2 * (tile - 1 - (k0 + lane * LB + i)));
-          }
-#pragma unroll
-          for (int i = 0; i < LB; ++i)
-            if (fl[i] == 0 && lane <= kp0) fl[i] = decode_seg<S>(sw[i], a.epoch, v[i]);
-          kp = lb_window<LB>(fl, resolved, whole);
-          if (resolved || whole) break;
-          ++it;
-          if (it == 8) t_wait = global_ns();  // first checked at it == 64
-          const bool stop = gave_up || it > SPIN_LIMIT ||
-                            ((it & 63u) == 0 && ((ld_relaxed_u32(a.err) & DEV_ERR_TIMEOUT) != 0u ||
-                                                 global_ns() - t_wait > WAIT_LIMIT_NS));
-          if (__any_sync(0xffffffffu, stop)) {
-            gave_up = true;
-            if (lane == 0) raise_error(a.err, DEV_ERR_TIMEOUT);
-#pragma unroll
-            for (int i = 0; i < LB; ++i)
-              if (fl[i] == 0) fl[i] = 2u;
-            kp = lb_window<LB>(fl, resolved, whole);
-            break;
-          }
-          __nanosleep(it < 4 ? 64 : (it < 16 ? 256 : 1024));  // back off: the predecessor is usually close behind
-        }
-        bool stop_here = false;
-        S lv = A::id();
-#pragma unroll
-        for (int i = 0; i < LB; ++i) {
-          if (!stop_here) lv = A::comb(v[i], lv);
-          stop_here = stop_here || fl[i] == 2u;
-        }
-        if (lane > kp) lv = A::id();
-        S wr = warp_reduce_rev<A>(lv);
-        wr = shfl_idx(wr, 0);
-        carry = A::comb(wr, carry);
-        if (resolved) break;
-        k0 += 32 * LB;
-      }
-      if (lane == 0 && ok) {
-        const S v = A::comb(carry, s_first_v);
-        out[s_first_id] = A::lower(a.has_seed ? A::comb(A::lift(z), v) : v);
-      }
-    }
-  }
+  finish(to_bits(s_tile_v), s_has_first ? to_bits(s_first_v) : 0, s_has_first && ok ? s_first_id : -1, s_tile_f != 0);
 }
 
 // One launcher per kernel instantiation, so that each gets its own
@@ -756,16 +822,21 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
 template <int OP, class T, int PREC, class OT>
 int launch_foldseg_tile(const CUtensorMap &tin, const SegTileArgs &a, int64_t ntiles, cudaStream_t s) {
   constexpr int FT_RPT = ft_rpt<typename Acc<OP, T, PREC>::S>();
-  const size_t smem = (size_t)FT_RPT * FT_THREADS * FT_ROW_BYTES + 1024;
+  const size_t tile = (size_t)FT_RPT * FT_THREADS * FT_ROW_BYTES + 1024;
+  const size_t all = (size_t)(FT_PER * FT_THREADS + FT_THREADS / 32) * sizeof(OT);  // small: the offsets, the warps' sums
+  const size_t smem = tile + (a.small ? all : 0);
   auto kern = foldseg_tile_kernel<OP, T, PREC, OT>;
   static std::atomic<uint64_t> attr_done{0};
-  smem_attrs_once(kern, (int)smem, attr_done);
+  smem_attrs_once(kern, (int)(tile + all), attr_done);
   kern<<<(unsigned)ntiles, FT_THREADS, smem, s>>>(tin, a);
+  const int st = check_launch();
+  if (st || a.small) return st;
+  foldseg_fix<OP, T, PREC><<<(unsigned)cdiv_h(ntiles, 256), 256, 0, s>>>(a);
   return check_launch();
 }
 
 template <int OP, class T, int PREC>
-int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, T *out, int64_t inner,
+int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bool lengths, T *out, int64_t inner,
                        int64_t nseg, bool has_seed, uint64_t seed, cudaStream_t s, bool *taken) {
   constexpr int ITEMS = FT_ROW_BYTES / sizeof(T);
   constexpr int FT_RPT = ft_rpt<typename Acc<OP, T, PREC>::S>();
@@ -781,26 +852,28 @@ int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, T 
   const int64_t ntiles = inner / TE + 1;
   if (ntiles * FT_RPT * FT_THREADS >= (1ll << 31)) return ACC_OK;  // TMA row coordinates are 32-bit
   if (nseg + 2 >= (1ll << TIDX_SHIFT)) return ACC_OK;
+  const bool small = nseg <= FT_SMALL && ntiles <= 2 * (int64_t)device_info().sms;
+  if (lengths && !small) return ACC_OK;  // the caller scans the lengths first
   *taken = true;
-  int st = ws_status(w, (size_t)ntiles * 2);
+  const size_t slot_bytes = (size_t)ntiles * sizeof(SegSlot);
+  int st = ws_scratch(w, slot_bytes + (size_t)(ntiles + 1) * sizeof(uint64_t));
   if (st) return st;
-  st = ws_scratch(w, (size_t)(ntiles + 1) * sizeof(uint64_t));
-  if (st) return st;
+  uint64_t *tidx = reinterpret_cast<uint64_t *>(static_cast<char *>(w->scratch) + slot_bytes);
   SegTileArgs a{};
   a.in = in; a.off = off; a.out = out;
   a.n = inner; a.nseg = nseg;
   a.full_rows = full_rows; a.ntiles = ntiles;
   a.seed = seed; a.has_seed = has_seed;
-  a.tidx = static_cast<const uint64_t *>(w->scratch);
-  a.status = w->status;
-  a.ticket = w->words + W_TICKET;
+  a.slots = static_cast<SegSlot *>(w->scratch);
+  a.tidx = tidx;
+  a.small = small ? (lengths ? 2 : 1) : 0;
+  a.done = w->words + W_DONE;
   a.err = w->words + W_ERR;
   a.epoch = ws_next_epoch(w, s);
-  {
+  if (!small) {
     const Device &d = device_info();
     int64_t pb = cdiv_h(nseg + 2, 256);
     if (pb > (int64_t)d.sms * 8) pb = (int64_t)d.sms * 8;
-    uint64_t *tidx = static_cast<uint64_t *>(w->scratch);
     if (off64)
       foldseg_tile_index<int64_t><<<(unsigned)pb, 256, 0, s>>>(static_cast<const int64_t *>(off), nseg, ntiles, TE,
                                                                 tidx, a.epoch);
@@ -856,9 +929,11 @@ int foldseg_typed(Workspace *w, const T *in, const void *off, int off64, T *out,
   return check_launch();
 }
 
+// `lengths`: `off` holds the segments' lengths; *taken says whether the call
+// was made (one launch scans them too), and nothing else is tried.
 int foldseg_dispatch(Workspace *w, int op, int type, int prec, const void *in, const void *off,
                      int off64, void *out, int64_t outer, int64_t inner, int64_t nseg,
-                     const void *seed, cudaStream_t s) {
+                     const void *seed, cudaStream_t s, bool lengths = false, bool *lengths_taken = nullptr) {
   return with_type(type, [&](auto tv) -> int {
     using T = decltype(tv);
     const uint64_t sb = seed_bits<T>(seed);
@@ -872,11 +947,13 @@ int foldseg_dispatch(Workspace *w, int op, int type, int prec, const void *in, c
             getenv("ACC_GB300_FOLDSEG") && strcmp(getenv("ACC_GB300_FOLDSEG"), "segments") == 0;
         if (outer == 1 && !per_segment) {
           bool taken = false;
-          const int st = foldseg_tile_typed<OP, T, P>(w, static_cast<const T *>(in), off, off64,
+          const int st = foldseg_tile_typed<OP, T, P>(w, static_cast<const T *>(in), off, off64, lengths,
                                                       static_cast<T *>(out), inner, nseg, seed != nullptr, sb, s,
                                                       &taken);
+          if (lengths) *lengths_taken = taken;
           if (taken || st) return st;
         }
+        if (lengths) return ACC_OK;
         return foldseg_typed<OP, T, P>(w, static_cast<const T *>(in), off, off64, static_cast<T *>(out),
                                        outer, inner, nseg, seed != nullptr, sb, s);
       });
@@ -921,14 +998,18 @@ extern "C" int acc_fold_seg_lengths(int op, int type, int prec, const void *in, 
   Workspace *w = workspace(s, &st);
   if (!w) return st;
   std::lock_guard<std::mutex> lk(w->mu);
+  bool taken = false;
+  st = foldseg_dispatch(w, op, type, prec, in, lengths, length_type == ACC_I64, out, outer, inner, nseg, seed, s, true,
+                        &taken);
+  if (taken || st) return st;
   // The offsets live at the END of the scratch area.  The front part,
   // list_bytes, holds what the fold itself keeps in scratch: the per-segment
   // path's long-segment list (at most inner / LONG_SEG + 1 entries) or the
-  // tiled path's tile index (inner / tile + 2 entries, tiles of >= 4096
+  // tiled path's slots and tile index (40 bytes per tile of at least 8192
   // values), both within list_bytes, so neither grows (and moves) the
   // scratch under the offsets.
   const size_t esz = length_type == ACC_I64 ? 8 : 4;
-  const size_t list_bytes = (size_t)(inner / LONG_SEG + 2) * sizeof(int64_t) + 256;
+  const size_t list_bytes = (size_t)(inner / LONG_SEG + 2) * 2 * sizeof(int64_t) + 512;
   const size_t off_bytes = (size_t)(nseg + 1) * esz;
   st = ws_scratch(w, list_bytes + off_bytes + 256);
   if (st) return st;
