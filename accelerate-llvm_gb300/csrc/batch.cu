@@ -4,18 +4,12 @@
 // The reference launches every skeleton separately, each with host-side
 // set-up (PTX/Execute.hs:835-881); thousands of small and medium requests are
 // dominated by launch latency.  Here a plan flattens a batch into work items
-// (request, tile), each request cut into tiles of NT x IPT elements; the
-// autotuner picks the launch shape (NT threads per CTA: 128, 256 or 512) and
-// the tile shape (IPT elements per thread) per (kind, type, size bucket), and
-// a batch runs with the NT preferred by most of its bytes.  One persistent
-// kernel draws items from an atomic ticket in table order:
-//   * fold tiles reduce their chunk (16-byte vector loads); the last tile of
-//     a request (per-request atomic ticket) folds the tile partials in order
-//     and writes z `f` result;
-//   * scan tiles stage their chunk in shared memory, scan it, and take the
-//     prefix of the earlier tiles of the same request by decoupled look-back
-//     (items are drawn in order, so every predecessor tile belongs to a
-//     running CTA).
+// (request, tile), each request cut into tiles of NT x IPT elements (scans) or
+// up to B_FOLD_STEPS such steps (folds); the autotuner picks the launch shape
+// (NT threads per CTA: 128, 256 or 512) and the tile shape (IPT elements per
+// thread) per (kind, type, size bucket), and a batch runs with the NT preferred
+// by most of its bytes.  One persistent kernel draws items from an atomic
+// ticket in table order; its design is at batch_kernel below.
 // All scratch is owned by the plan and allocated when the plan is made; a
 // launch allocates nothing and takes its look-back epoch from a device word
 // that the last CTA advances, so a captured graph replays unchanged.
@@ -35,7 +29,8 @@
 namespace accgb {
 
 constexpr int BT = 256;                    // threads per CTA of untuned launches and of the serving arena
-constexpr int B_MAX_TILE_BYTES = 32768;    // largest tile staged in shared memory
+constexpr int B_FOLD_STEPS = 4;            // tiles' worth of elements in one fold item
+constexpr int B_BYTES[2] = {16, 64};       // bytes of a tile per thread, the two tile shapes
 
 struct BReq {
   const void *in;
@@ -66,8 +61,7 @@ __device__ __forceinline__ void b_publish(uint64_t *status, int64_t t, uint32_t 
   st_relaxed_u64(status + 2 * t, tag | (b & 0xffffffffull));
 }
 template <class S>
-__device__ __forceinline__ uint32_t b_peek(const uint64_t *status, int64_t t, uint32_t epoch, S &v) {
-  const SlotWords s = ld_slot(status + 2 * t);  // both words in one access
+__device__ __forceinline__ uint32_t b_decode(SlotWords s, uint32_t epoch, S &v) {
   const uint32_t tag = (uint32_t)(s.w0 >> 32);
   if ((tag >> 2) != epoch) return 0;
   uint64_t b = s.w0 & 0xffffffffull;
@@ -79,252 +73,431 @@ __device__ __forceinline__ uint32_t b_peek(const uint64_t *status, int64_t t, ui
   return tag & 3u;
 }
 
-// CTA-wide ordered reduction (valid in thread 0).
-template <class A, int NT>
-__device__ __forceinline__ typename A::S b_block_reduce(typename A::S v, typename A::S *s_part) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  v = warp_reduce<A>(v);
-  if (lane == 0) s_part[warp] = v;
-  __syncthreads();
-  if (warp == 0) {
-    v = lane < NT / 32 ? s_part[lane] : A::id();
-    v = warp_reduce<A>(v);
+enum { BK_FOLD = 0, BK_SCAN = 1 };
+
+// An item as the CTA sees it: its request and its place in it.
+struct __align__(16) BDesc {
+  BReq q;
+  int64_t item;  // -1: no more items
+  int32_t r, pad;
+};
+static_assert(sizeof(BReq) == 64, "a request's descriptor is four 16-byte words");
+
+template <int OP, class T> constexpr int b_prec() {
+  return OP == ACC_ADD && std::is_same<T, float>::value ? PREC_COMP : PREC_PLAIN;
+}
+// f(T{}) for the request's element type (I32, I64, F32, F64)
+template <class F> __device__ __forceinline__ void b_with_type(int type, F &&f) {
+  switch (type) {
+    case ACC_I32: f(int32_t{}); break;
+    case ACC_I64: f(int64_t{}); break;
+    case ACC_F32: f(float{}); break;
+    default: f(double{}); break;
   }
-  __syncthreads();
-  return v;
 }
 
-template <int OP, class T, int PREC, int NT>
-__device__ void b_fold_tile(const BatchArgs &a, const BReq &q, int64_t item, int32_t r, unsigned char *smem) {
-  using A = Acc<OP, T, PREC>;
-  using S = typename A::S;
-  __shared__ bool s_last;
-  S *s_part = reinterpret_cast<S *>(smem);
-  const int64_t tile = item - q.first_item;
-  const int64_t ts = (int64_t)q.ipt * NT;
-  const int64_t b = tile * ts;
-  const int64_t e = b + ts < q.n ? b + ts : q.n;
-  const T *src = static_cast<const T *>(q.in) + b;
-  const int64_t len = e - b;
-  // 16-byte vector body, scalar head and tail.
-  constexpr int VEC = 16 / sizeof(T);
-  S acc = A::id();
-  const uintptr_t addr = reinterpret_cast<uintptr_t>(src);
-  int64_t head = (int64_t)(((16u - (addr & 15u)) & 15u) / sizeof(T));
-  if (head > len) head = len;
-  if ((int64_t)threadIdx.x < head) acc = A::push(acc, src[threadIdx.x]);
-  const int64_t nvec = (len - head) / VEC;
-  const uint4 *qv = reinterpret_cast<const uint4 *>(src + head);
-  for (int64_t i = threadIdx.x; i < nvec; i += NT) {
-    uint4 v = ld_stream16(qv + i);
-    T el[VEC];
-    memcpy(el, &v, 16);
+// A compute thread's part of a tile, raw: 16 words, of which a tile of 16
+// bytes per thread uses four.  A warp's part is 32 x ipt consecutive elements,
+// read coalesced: element j * 32 + lane of the part is word(s) j.
+struct BRaw { uint32_t w[16]; };
+
+template <class W, int N>
+__device__ __forceinline__ void b_load_words(const W *p, int64_t left, BRaw &raw) {
 #pragma unroll
-    for (int k = 0; k < VEC; ++k) acc = A::push(acc, el[k]);
-  }
-  const int64_t tail0 = head + nvec * VEC;
-  if (tail0 + threadIdx.x < len) acc = A::push(acc, src[tail0 + threadIdx.x]);
-  acc = b_block_reduce<A, NT>(acc, s_part);
-  // One 8-byte slot per item whatever the state's size, so that requests of
-  // different types in one batch never share partial slots.
-  static_assert(sizeof(S) <= sizeof(uint64_t), "fold state larger than a partial slot");
-  auto part = [&](int64_t it) { return reinterpret_cast<S *>(a.partials + it); };
-  if (threadIdx.x == 0) {
-    *part(item) = acc;
-    __threadfence();
-    const uint32_t prev = atomicAdd(a.req_ticket + r, 1u);
-    s_last = prev == (uint32_t)(q.ntiles - 1);
-  }
-  __syncthreads();
-  if (s_last) {
-    __threadfence();
-    S v = A::id();
-    const int64_t per = (q.ntiles + NT - 1) / NT;
-    const int64_t lo = threadIdx.x * per, hi = lo + per < q.ntiles ? lo + per : q.ntiles;
-    for (int64_t i = lo; i < hi; ++i) v = A::comb(v, ld_state<S>(part(q.first_item + i)));
-    v = b_block_reduce<A, NT>(v, s_part);
-    if (threadIdx.x == 0) {
-      if (q.has_seed) v = A::comb(A::lift(from_bits<T>(q.seed)), v);
-      *static_cast<T *>(q.out) = A::lower(v);
-      a.req_ticket[r] = 0u;  // re-arm for the next launch
+  for (int j = 0; j < N; ++j)
+    if (j * 32 < left) {
+      const W v = p[j * 32];
+      memcpy(&raw.w[j * (sizeof(W) / 4)], &v, sizeof(W));
     }
+}
+// Elements [at, at + 32 ipt) of the request, from lane's first one (at + lane).
+__device__ __forceinline__ void b_load(const BReq &q, int64_t at, BRaw &raw) {
+  const int64_t left = q.n - at;
+  if (q.type == ACC_I32 || q.type == ACC_F32) {
+    const uint32_t *p = static_cast<const uint32_t *>(q.in) + at;
+    if (q.ipt == 16) b_load_words<uint32_t, 16>(p, left, raw);
+    else b_load_words<uint32_t, 4>(p, left, raw);
+  } else {
+    const uint64_t *p = static_cast<const uint64_t *>(q.in) + at;
+    if (q.ipt == 8) b_load_words<uint64_t, 8>(p, left, raw);
+    else b_load_words<uint64_t, 2>(p, left, raw);
   }
-  __syncthreads();
+}
+template <class T> __device__ __forceinline__ T b_elem(const BRaw &raw, int j) {
+  T x;
+  memcpy(&x, &raw.w[j * (sizeof(T) / 4)], sizeof(T));
+  return x;
 }
 
-template <int OP, class T, int PREC, int IPT, int NT>
-__device__ void b_scan_tile(const BatchArgs &a, const BReq &q, int64_t item, uint32_t epoch, unsigned char *smem) {
-  using A = Acc<OP, T, PREC>;
+// Scan, first pass: the warp turns its part in shared memory into K consecutive
+// elements per lane (rows of an odd pitch) and scans the lanes' sums.  Returns
+// the state of the lanes before this one; `sum` is the warp's.
+template <int OP, class T, int K>
+__device__ __forceinline__ uint64_t b_scan_pass1(const BRaw &raw, int64_t left, unsigned char *wbuf, uint64_t &sum) {
+  using A = Acc<OP, T, b_prec<OP, T>()>;
   using S = typename A::S;
-  __shared__ S s_warp[NT / 32];
-  __shared__ S s_prefix;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  constexpr int ipt = IPT;  // compile time: the staging index math is shifts and masks
-  constexpr int pitch = ipt + 1;  // padded row: conflict-free thread-per-row access
-  T *tile_s = reinterpret_cast<T *>(smem + 256);
-  const int64_t tile = item - q.first_item;
-  const int64_t ts = (int64_t)ipt * NT;
-  const int64_t b = tile * ts;
-  const T idT = Prim<OP, T>::id();
-  const T *src = static_cast<const T *>(q.in);
-  for (int k = tid; k < ts; k += NT) {
-    const int64_t gi = b + k;
-    tile_s[(k / ipt) * pitch + (k % ipt)] = gi < q.n ? src[gi] : idT;
-  }
-  __syncthreads();
-  T *row = tile_s + tid * pitch;
+  const int lane = threadIdx.x & 31;
+  T *turn = reinterpret_cast<T *>(wbuf) + (lane / K) * (K + 1) + lane % K;
+  const T *row = reinterpret_cast<const T *>(wbuf) + lane * (K + 1);
+#pragma unroll
+  for (int j = 0; j < K; ++j) turn[j * (32 / K) * (K + 1)] = j * 32 < left ? b_elem<T>(raw, j) : Prim<OP, T>::id();
+  __syncwarp();
   S agg = A::lift(row[0]);
 #pragma unroll
-  for (int j = 1; j < ipt; ++j) agg = A::push(agg, row[j]);
-  S incl = warp_scan_incl<A>(agg);
-  S up = shfl_up(incl, 1);
-  const S excl_lane = lane == 0 ? A::id() : up;
-  if (lane == 31) s_warp[warp] = incl;
-  __syncthreads();
-  S wpre = A::id();
-  for (int w = 0; w < warp; ++w) wpre = A::comb(wpre, s_warp[w]);
-  if (warp == 0) {
-    S bagg = s_warp[0];
-    for (int w = 1; w < NT / 32; ++w) bagg = A::comb(bagg, s_warp[w]);
-    S prefix = q.has_seed ? A::lift(from_bits<T>(q.seed)) : A::id();
-    if (tile > 0) {
-      if (lane == 0) b_publish<S>(a.status, item, epoch, 1u, bagg);
-      S acc = A::id();
-      int64_t k0 = 0;
-      bool gave_up = false;
-      while (true) {
-        const int64_t d = k0 + lane;
-        const bool exists = d < tile;  // predecessors of the same request only
-        const int64_t pt = item - 1 - d;
-        uint32_t flag = exists ? 0u : 2u;
-        S v = A::id();
-        uint32_t it = 0;
-        uint64_t t_wait = 0;
-        while (true) {
-          if (exists && flag == 0) flag = b_peek<S>(a.status, pt, epoch, v);
-          if (__all_sync(0xffffffffu, flag != 0)) break;
-          ++it;
-          if (it == 8) t_wait = global_ns();  // first checked at it == 64
-          const bool stop = gave_up || it > SPIN_LIMIT ||
-                            ((it & 63u) == 0 && ((ld_relaxed_u32(a.words) & DEV_ERR_TIMEOUT) != 0u ||
-                                                 global_ns() - t_wait > WAIT_LIMIT_NS));
-          if (__any_sync(0xffffffffu, stop)) {
-            gave_up = true;
-            if (lane == 0) raise_error(a.words, DEV_ERR_TIMEOUT);
-            if (flag == 0) flag = 2u;
-            break;
-          }
-          __nanosleep(it < 8 ? 32 : 128);
-        }
-        const unsigned pm = __ballot_sync(0xffffffffu, flag == 2u);
-        const int kp = pm ? __ffs(pm) - 1 : 32;
-        if (lane > kp) v = A::id();
-        S wv = warp_reduce_rev<A>(v);
-        wv = shfl_idx(wv, 0);
-        acc = A::comb(wv, acc);
-        if (pm) break;
-        k0 += 32;
-      }
-      prefix = acc;  // the seed already sits in the request's first tile
-    }
-    if (lane == 0) {
-      b_publish<S>(a.status, item, epoch, 2u, A::comb(prefix, bagg));
-      s_prefix = prefix;
-    }
-  }
-  __syncthreads();
-  S run = A::comb(s_prefix, A::comb(wpre, excl_lane));
+  for (int j = 1; j < K; ++j) agg = A::push(agg, row[j]);
+  const S incl = warp_scan_incl<A>(agg);
+  const S up = shfl_up(incl, 1);
+  sum = to_bits(shfl_idx(incl, 31));
+  return to_bits(lane == 0 ? A::id() : up);
+}
+// Scan, second pass: rescan from the state before this lane and store.
+template <int OP, class T, int K>
+__device__ __forceinline__ void b_scan_pass2(const BReq &q, int64_t at, unsigned char *wbuf, uint64_t before) {
+  using A = Acc<OP, T, b_prec<OP, T>()>;
+  const int lane = threadIdx.x & 31;
+  T *row = reinterpret_cast<T *>(wbuf) + lane * (K + 1);
+  const T *turn = reinterpret_cast<const T *>(wbuf) + (lane / K) * (K + 1) + lane % K;
+  typename A::S run = from_bits<typename A::S>(before);
 #pragma unroll
-  for (int j = 0; j < ipt; ++j) {
+  for (int j = 0; j < K; ++j) {
     run = A::push(run, row[j]);
     row[j] = A::lower(run);
   }
-  __syncthreads();
-  T *dst = static_cast<T *>(q.out);
-  for (int k = tid; k < ts; k += NT) {
-    const int64_t gi = b + k;
-    if (gi < q.n) dst[gi] = tile_s[(k / ipt) * pitch + (k % ipt)];
-  }
-  __syncthreads();
+  __syncwarp();
+  T *to = static_cast<T *>(q.out) + at;
+  const int64_t left = q.n - at;
+#pragma unroll
+  for (int j = 0; j < K; ++j)
+    if (j * 32 < left) to[j * 32] = turn[j * (32 / K) * (K + 1)];
+  __syncwarp();
 }
 
-// Scan tiles are instantiated per elements-per-thread (powers of two up to
-// the 32 KiB tile limit for NT threads), picked by the tile's planned value.
-template <int OP, class T, int PREC, int NT>
-__device__ __forceinline__ void b_scan_tile_any(const BatchArgs &a, const BReq &q, int64_t item, uint32_t epoch,
-                                                unsigned char *smem) {
-  constexpr int MAXI = B_MAX_TILE_BYTES / (NT * (int)sizeof(T));
-  switch (q.ipt) {
-    case 1: b_scan_tile<OP, T, PREC, 1, NT>(a, q, item, epoch, smem); break;
-    case 2: b_scan_tile<OP, T, PREC, 2, NT>(a, q, item, epoch, smem); break;
-    case 4: b_scan_tile<OP, T, PREC, 4, NT>(a, q, item, epoch, smem); break;
-    case 8: b_scan_tile<OP, T, PREC, 8, NT>(a, q, item, epoch, smem); break;
-    default:
-      if constexpr (MAXI >= 64) {
-        if (q.ipt == 64) { b_scan_tile<OP, T, PREC, 64, NT>(a, q, item, epoch, smem); break; }
-      }
-      if constexpr (MAXI >= 32) {
-        if (q.ipt == 32) { b_scan_tile<OP, T, PREC, 32, NT>(a, q, item, epoch, smem); break; }
-      }
-      if constexpr (MAXI >= 16) b_scan_tile<OP, T, PREC, 16, NT>(a, q, item, epoch, smem);
-      else b_scan_tile<OP, T, PREC, 8, NT>(a, q, item, epoch, smem);
-      break;
-  }
-}
-
-enum { BK_FOLD = 0, BK_SCAN = 1 };
-
-// The register budget: ~51 per thread with 256 or 512 threads (1,280 threads
-// per SM), 64 with 128 threads (1,024 per SM; 48 would spill).
-template <int OP, int NT>
-__global__ void __launch_bounds__(NT, NT == 128 ? 8 : 1280 / NT) batch_kernel(BatchArgs a) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int64_t s_item;
-  __shared__ BReq s_req;
-  __shared__ uint32_t s_epoch;
-  if (threadIdx.x == 0) s_epoch = (ld_relaxed_u32(a.words + 2) & ((1u << 29) - 1)) + 1;
-  const uint32_t last_ticket = (uint32_t)a.nitems + gridDim.x - 1;
+// The service warp's look-back: the combination of every earlier tile of the
+// request, from the nearest published inclusive prefix on (warp-collective), in
+// windows of 32 x B_LOOK tiles whose slots are loaded at once (1000 requests,
+// 256 threads: one slot per lane 0.652 ms, two 0.669, four 0.700: a window
+// waits for every tile in it up to the prefix).
+constexpr int B_LOOK = 1;
+template <class A>
+__device__ __forceinline__ typename A::S b_lookback(const BatchArgs &a, int64_t item, int64_t tile, uint32_t epoch) {
+  using S = typename A::S;
+  const int lane = threadIdx.x & 31;
+  S acc = A::id();
+  int64_t k0 = 0;
+  bool gave_up = false;
   while (true) {
-    if (threadIdx.x == 0) {
-      const uint32_t t = atomicAdd(a.words + 1, 1u);
-      if (t == last_ticket) {
-        // Every CTA has drawn its last ticket (and read the epoch): re-arm the
-        // ticket and advance the epoch for the next launch or graph replay.
-        a.words[1] = 0u;
-        atomicAdd(a.words + 2, 1u);
-      }
-      s_item = (int64_t)t < a.nitems ? (int64_t)t : -1;
-      if (s_item >= 0) s_req = a.reqs[a.item_req[s_item]];
+    uint32_t fl[B_LOOK];
+    S v[B_LOOK];
+#pragma unroll
+    for (int i = 0; i < B_LOOK; ++i) {
+      fl[i] = k0 + lane * B_LOOK + i < tile ? 0u : 2u;  // predecessors of the same request only
+      v[i] = A::id();
     }
-    __syncthreads();
-    const int64_t item = s_item;
-    if (item < 0) break;
-    const BReq q = s_req;
-    const int32_t r = a.item_req[item];
-    const uint32_t epoch = s_epoch;
-    if (q.kind == BK_FOLD) {
-      switch (q.type) {
-        case ACC_I32: b_fold_tile<OP, int32_t, 0, NT>(a, q, item, r, smem); break;
-        case ACC_I64: b_fold_tile<OP, int64_t, 0, NT>(a, q, item, r, smem); break;
-        case ACC_F32: b_fold_tile<OP, float, OP == ACC_ADD ? PREC_COMP : PREC_PLAIN, NT>(a, q, item, r, smem); break;
-        default: b_fold_tile<OP, double, 0, NT>(a, q, item, r, smem); break;
+    uint32_t it = 0;
+    uint64_t t_wait = 0;
+    bool resolved = false, whole = false;
+    int kp = 32;
+    while (true) {
+      const int kp0 = lb_stop_lane<B_LOOK>(fl);
+      SlotWords sw[B_LOOK];
+#pragma unroll
+      for (int i = 0; i < B_LOOK; ++i) {
+        sw[i] = SlotWords{0ull, 0ull};
+        if (fl[i] == 0 && lane <= kp0) sw[i] = ld_slot(a.status + 2 * (item - 1 - (k0 + lane * B_LOOK + i)));
       }
+#pragma unroll
+      for (int i = 0; i < B_LOOK; ++i)
+        if (fl[i] == 0 && lane <= kp0) fl[i] = b_decode<S>(sw[i], epoch, v[i]);
+      kp = lb_window<B_LOOK>(fl, resolved, whole);
+      if (resolved || whole) break;
+      ++it;
+      if (it == 8) t_wait = global_ns();  // first checked at it == 64
+      const bool stop = gave_up || it > SPIN_LIMIT ||
+                        ((it & 63u) == 0 && ((ld_relaxed_u32(a.words) & DEV_ERR_TIMEOUT) != 0u ||
+                                             global_ns() - t_wait > WAIT_LIMIT_NS));
+      if (__any_sync(0xffffffffu, stop)) {
+        gave_up = true;
+        if (lane == 0) raise_error(a.words, DEV_ERR_TIMEOUT);
+#pragma unroll
+        for (int i = 0; i < B_LOOK; ++i)
+          if (fl[i] == 0) fl[i] = 2u;
+        kp = lb_window<B_LOOK>(fl, resolved, whole);
+        break;
+      }
+      __nanosleep(it < 8 ? 32 : 128);
+    }
+    // lane-local fold from the nearest predecessor outwards, up to the first prefix
+    bool seen = false;
+    S lv = A::id();
+#pragma unroll
+    for (int i = 0; i < B_LOOK; ++i) {
+      if (!seen) lv = A::comb(v[i], lv);
+      seen = seen || fl[i] == 2u;
+    }
+    if (lane > kp) lv = A::id();
+    acc = A::comb(shfl_idx(warp_reduce_rev<A>(lv), 0), acc);
+    if (resolved) break;
+    k0 += 32 * B_LOOK;
+  }
+  return acc;
+}
+
+// The persistent kernel.  NT compute threads and one service warp per CTA, which
+// hand items over through mbarriers:
+//   * the service warp draws the next item and fetches its descriptor while the
+//     compute warps work on this one, looks back for scan tiles, and finishes
+//     folds (one partial per item, the last item of a request folds them in
+//     order);
+//   * the compute warps keep the next tile's loads in flight in registers while
+//     they work on one.  A scan tile takes two passes: its second, from the
+//     prefix that the service warp found, runs after the first pass of the
+//     CTA's next item, so that a look-back overlaps that.
+// An item waits only on items with smaller tickets, which running CTAs hold and
+// work through in order, so the smallest unfinished one can always finish.
+// Every wait is bounded; a warp whose wait ran out raises DEV_ERR_TIMEOUT and
+// returns (so do the others, in turn).
+// Bound: the latency of a scan tile's look-back, then issue.  Measured on a
+// GB300, 1000 requests of 2^8 .. 2^22 elements, folds and scans of Int32 and
+// Float32 (floor 0.347 ms), against one tile at a time per CTA, loaded, scanned,
+// looked back for and stored between barriers: 1.20 -> 0.60 ms (512 threads; 256:
+// 0.64).  A tile's sum published by the service warp, after the look-back of the
+// item before: 2.6 ms.  Tickets drawn five items ahead: 0.90 ms (a CTA's queue
+// holds back the tiles that others wait for).  Fold items of 1 / 2 / 4 / 8 steps
+// (256 threads): 0.713 / 0.651 / 0.637 / 0.669 ms.
+constexpr int B_RING = 8;   // descriptors
+constexpr int B_KEEP = 4;   // items whose warp totals and prefixes are kept
+
+// bytes of a warp's buffer (32 rows of 64 bytes and one element), for one tile
+__host__ __device__ constexpr int b_wbuf_bytes() { return 32 * (64 + 8); }
+
+template <int OP, int NT>
+__global__ void __launch_bounds__(NT + 32, NT == 128 ? 6 : NT == 256 ? 4 : 2) batch_kernel(BatchArgs a) {
+  constexpr int NW = NT / 32;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ BDesc s_desc[B_RING];
+  __shared__ uint64_t s_warp[B_KEEP][NW];  // states as bits
+  __shared__ uint64_t s_sum[B_KEEP], s_prefix[B_KEEP];
+  __shared__ uint32_t s_epoch;
+  __shared__ int s_warps[B_KEEP];  // compute warps that have an item's sum
+  __shared__ uint64_t b_desc[B_RING], b_sum[2], b_done[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) {
+    for (int i = 0; i < B_RING; ++i) mbar_init(&b_desc[i], 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&b_sum[i], 1);
+      mbar_init(&b_done[i], 1);
+    }
+    for (int i = 0; i < B_KEEP; ++i) s_warps[i] = 0;
+    s_epoch = (ld_relaxed_u32(a.words + 2) & ((1u << 29) - 1)) + 1;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  const uint32_t epoch = s_epoch;
+  auto wait = [&](uint64_t *bar, int64_t phase) -> bool {  // warp-uniform
+    return __all_sync(0xffffffffu, mbar_wait_flagged(bar, (uint32_t)phase & 1u, a.words));
+  };
+
+  if (warp == NW) {
+    // ---- service warp
+    const uint32_t last_ticket = (uint32_t)a.nitems + gridDim.x - 1;
+    // Draw the item of index i and hand it to the compute warps.  The holder of
+    // the last ticket knows that every CTA has drawn its last one (and read the
+    // epoch): it re-arms the ticket and advances the epoch for the next launch or
+    // graph replay.
+    auto claim = [&](int64_t i) {
+      int64_t item = -1;
+      if (lane == 0) {
+        const uint32_t t = atomicAdd(a.words + 1, 1u);
+        if (t == last_ticket) {
+          a.words[1] = 0u;
+          atomicAdd(a.words + 2, 1u);
+        }
+        if ((int64_t)t < a.nitems) item = t;
+      }
+      item = __shfl_sync(0xffffffffu, item, 0);
+      BDesc &d = s_desc[i & (B_RING - 1)];
+      if (item >= 0) {
+        const int32_t r = a.item_req[item];
+        if (lane < 4) reinterpret_cast<uint4 *>(&d.q)[lane] = reinterpret_cast<const uint4 *>(a.reqs + r)[lane];
+        if (lane == 0) d.r = r;
+      }
+      if (lane == 0) d.item = item;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&b_desc[i & (B_RING - 1)]);
+    };
+    claim(0);
+    for (int64_t i = 0;; ++i) {
+      if (s_desc[i & (B_RING - 1)].item < 0) break;
+      claim(i + 1);
+      if (!wait(&b_sum[i & 1], i >> 1)) return;
+      const BDesc &d = s_desc[i & (B_RING - 1)];
+      const int64_t item = d.item, tile = item - d.q.first_item;
+      const uint64_t sum_bits = s_sum[i & (B_KEEP - 1)];
+      b_with_type(d.q.type, [&](auto tv) {
+        using T = decltype(tv);
+        using A = Acc<OP, T, b_prec<OP, T>()>;
+        using S = typename A::S;
+        const S sum = from_bits<S>(sum_bits);
+        const S z = A::lift(from_bits<T>(d.q.seed));
+        if (d.q.kind == BK_SCAN) {
+          S prefix = d.q.has_seed ? z : A::id();  // of the request's first tile
+          if (tile > 0) prefix = b_lookback<A>(a, item, tile, epoch);
+          if (lane == 0) {
+            if (tile + 1 < d.q.ntiles) b_publish<S>(a.status, item, epoch, 2u, A::comb(prefix, sum));
+            s_prefix[i & (B_KEEP - 1)] = to_bits(prefix);
+          }
+        } else if (d.q.ntiles == 1) {
+          if (lane == 0) *static_cast<T *>(d.q.out) = A::lower(d.q.has_seed ? A::comb(z, sum) : sum);
+        } else {
+          // One 8-byte slot per item whatever the state's size, so that requests
+          // of different types in one batch never share partial slots.
+          auto part = [&](int64_t k) { return reinterpret_cast<S *>(a.partials + k); };
+          uint32_t prev = 0;
+          if (lane == 0) {
+            *part(item) = sum;
+            __threadfence();
+            prev = atomicAdd(a.req_ticket + d.r, 1u);
+          }
+          if (__shfl_sync(0xffffffffu, prev, 0) == (uint32_t)(d.q.ntiles - 1)) {
+            __threadfence();
+            const int64_t per = (d.q.ntiles + 31) / 32;
+            const int64_t lo = lane * per, hi = lo + per < d.q.ntiles ? lo + per : d.q.ntiles;
+            S v = A::id();
+            for (int64_t k = lo; k < hi; ++k) v = A::comb(v, ld_state<S>(part(d.q.first_item + k)));
+            v = warp_reduce<A>(v);
+            if (lane == 0) {
+              *static_cast<T *>(d.q.out) = A::lower(d.q.has_seed ? A::comb(z, v) : v);
+              a.req_ticket[d.r] = 0u;  // re-arm for the next launch
+            }
+          }
+        }
+      });
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&b_done[i & 1]);
+    }
+    return;
+  }
+
+  // ---- compute warps
+  unsigned char *wbufs = smem + warp * (2 * b_wbuf_bytes());
+  auto part_of = [&](const BDesc &d) -> int64_t {  // this lane's first element of the item
+    const int64_t tile = d.item - d.q.first_item;
+    const int64_t ts = (int64_t)d.q.ipt * NT * (d.q.kind == BK_FOLD ? B_FOLD_STEPS : 1);
+    return tile * ts + warp * (32 * d.q.ipt) + lane;
+  };
+  auto pass2 = [&](int64_t i, uint64_t before) -> bool {
+    if (!wait(&b_done[i & 1], i >> 1)) return false;
+    const BDesc &d = s_desc[i & (B_RING - 1)];
+    if (d.q.kind != BK_SCAN) return true;
+    unsigned char *wbuf = wbufs + (i & 1) * b_wbuf_bytes();
+    const uint64_t *totals = s_warp[i & (B_KEEP - 1)];
+    const uint64_t prefix = s_prefix[i & (B_KEEP - 1)];
+    const int64_t at = part_of(d);
+    b_with_type(d.q.type, [&](auto tv) {
+      using T = decltype(tv);
+      using A = Acc<OP, T, b_prec<OP, T>()>;
+      using S = typename A::S;
+      constexpr int KW = 64 / sizeof(T), KN = 16 / sizeof(T);
+      S run = from_bits<S>(prefix);
+      for (int w = 0; w < warp; ++w) run = A::comb(run, from_bits<S>(totals[w]));
+      run = A::comb(run, from_bits<S>(before));
+      if (d.q.ipt == KW) b_scan_pass2<OP, T, KW>(d.q, at, wbuf, to_bits(run));
+      else b_scan_pass2<OP, T, KN>(d.q, at, wbuf, to_bits(run));
+    });
+    return true;
+  };
+  BRaw raw;
+  uint64_t before_prev = 0;
+  if (!wait(&b_desc[0], 0)) return;
+  if (s_desc[0].item < 0) return;
+  b_load(s_desc[0].q, part_of(s_desc[0]), raw);
+  for (int64_t i = 0;; ++i) {
+    const BDesc &d = s_desc[i & (B_RING - 1)], &dn = s_desc[(i + 1) & (B_RING - 1)];
+    const int64_t at = part_of(d);
+    uint64_t before = 0, sum = 0;
+    bool ok = true;
+    auto load_next = [&]() {
+      ok = wait(&b_desc[(i + 1) & (B_RING - 1)], (i + 1) / B_RING);
+      if (ok && dn.item >= 0) b_load(dn.q, part_of(dn), raw);
+    };
+    if (d.q.kind == BK_SCAN) {
+      unsigned char *wbuf = wbufs + (i & 1) * b_wbuf_bytes();
+      const int64_t left = d.q.n - at;
+      b_with_type(d.q.type, [&](auto tv) {
+        using T = decltype(tv);
+        constexpr int KW = 64 / sizeof(T), KN = 16 / sizeof(T);
+        before = d.q.ipt == KW ? b_scan_pass1<OP, T, KW>(raw, left, wbuf, sum) : b_scan_pass1<OP, T, KN>(raw, left, wbuf, sum);
+      });
     } else {
-      switch (q.type) {
-        case ACC_I32: b_scan_tile_any<OP, int32_t, 0, NT>(a, q, item, epoch, smem); break;
-        case ACC_I64: b_scan_tile_any<OP, int64_t, 0, NT>(a, q, item, epoch, smem); break;
-        case ACC_F32: b_scan_tile_any<OP, float, OP == ACC_ADD ? PREC_COMP : PREC_PLAIN, NT>(a, q, item, epoch, smem); break;
-        default: b_scan_tile_any<OP, double, 0, NT>(a, q, item, epoch, smem); break;
-      }
+      // the item's steps, the next one's loads in flight
+      const int64_t step = (int64_t)d.q.ipt * NT;
+      int64_t end = (d.item - d.q.first_item + 1) * step * B_FOLD_STEPS;
+      if (end > d.q.n) end = d.q.n;
+      b_with_type(d.q.type, [&](auto tv) {
+        using T = decltype(tv);
+        using A = Acc<OP, T, b_prec<OP, T>()>;
+        constexpr int KW = 64 / sizeof(T), KN = 16 / sizeof(T);
+        typename A::S acc = A::id();
+        for (int64_t e = at;; e += step) {
+          const BRaw cur = raw;
+          const int64_t left = d.q.n - e;
+          // uniform over the warp: whether any lane has elements in the next step
+          const bool more = e - lane + step < end;
+          if (more) b_load(d.q, e + step, raw);
+          if (d.q.ipt == KW) {
+#pragma unroll
+            for (int j = 0; j < KW; ++j)
+              if (j * 32 < left) acc = A::push(acc, b_elem<T>(cur, j));
+          } else {
+#pragma unroll
+            for (int j = 0; j < KN; ++j)
+              if (j * 32 < left) acc = A::push(acc, b_elem<T>(cur, j));
+          }
+          if (!more) break;
+        }
+        sum = to_bits(warp_reduce<A>(acc));
+      });
     }
-    __syncthreads();
+    // The warp that completes the item's sum hands it to the service warp, and
+    // publishes a scan tile's at once: the service warp may still be looking back
+    // for the item before, and later tiles must not wait for that.
+    int last = 0;
+    if (lane == 0) {
+      s_warp[i & (B_KEEP - 1)][warp] = sum;
+      __threadfence_block();
+      last = atomicAdd(&s_warps[i & (B_KEEP - 1)], 1) == NW - 1;
+    }
+    if (__shfl_sync(0xffffffffu, last, 0)) {
+      __threadfence_block();
+      b_with_type(d.q.type, [&](auto tv) {
+        using T = decltype(tv);
+        using A = Acc<OP, T, b_prec<OP, T>()>;
+        using S = typename A::S;
+        const S v = warp_reduce<A>(lane < NW ? from_bits<S>(s_warp[i & (B_KEEP - 1)][lane]) : A::id());
+        if (lane == 0) {
+          if (d.q.kind == BK_SCAN && d.item > d.q.first_item) b_publish<S>(a.status, d.item, epoch, 1u, v);
+          s_sum[i & (B_KEEP - 1)] = to_bits(v);
+          s_warps[i & (B_KEEP - 1)] = 0;
+          mbar_arrive(&b_sum[i & 1]);
+        }
+      });
+      __syncwarp();
+    }
+    load_next();
+    if (!ok) return;
+    if (i > 0 && !pass2(i - 1, before_prev)) return;
+    before_prev = before;
+    if (dn.item < 0) {
+      pass2(i, before);
+      return;
+    }
   }
 }
 
 // ---------------------------------------------------------------- autotuner table
 // Launch and tile shape per (kind, type, log2 size bucket): NT threads per CTA
-// and IPT elements per thread (a tile is NT x IPT elements).  Filled by
-// acc_batch_autotune, persisted as JSON.
+// and IPT elements per thread (a tile is NT x IPT elements), 16 or 64 bytes'
+// worth.  Filled by acc_batch_autotune, persisted as JSON.
 constexpr int B_NT[3] = {128, 256, 512};
 struct TuneKey {
   int kind, type, bucket;
@@ -338,15 +511,11 @@ static std::map<TuneKey, TuneVal> g_tune;
 
 static bool valid_nt(int nt) { return nt == 128 || nt == 256 || nt == 512; }
 static int type_bytes(int type) { return (type == ACC_I64 || type == ACC_F64) ? 8 : 4; }
-static int max_ipt(int type, int nt) { return B_MAX_TILE_BYTES / (nt * type_bytes(type)); }
-// Elements per thread as the kernel takes them: within [1, max_ipt], rounded
-// down to a power of two (scan tiles are instantiated for those only).
-static int norm_ipt(int ipt, int type, int nt) {
-  if (ipt < 1) ipt = 1;
-  if (ipt > max_ipt(type, nt)) ipt = max_ipt(type, nt);
-  int p = 1;
-  while (p * 2 <= ipt) p *= 2;
-  return p;
+// Elements per thread as the kernel takes them: 16 or 64 bytes' worth, the
+// nearer one.
+static int norm_ipt(int ipt, int type) {
+  const int eb = type_bytes(type);
+  return B_BYTES[ipt * eb > 32 ? 1 : 0] / eb;
 }
 static int bucket_of(int64_t n) {
   int b = 0;
@@ -354,18 +523,17 @@ static int bucket_of(int64_t n) {
   return b;
 }
 static int default_ipt(int kind, int type, int64_t n) {
-  // Before tuning (256 threads): one wave of small tiles for small requests,
-  // large tiles otherwise.
-  const int cap = max_ipt(type, BT);
-  int ipt = n <= (1 << 14) ? 4 : n <= (1 << 18) ? 8 : 16;
   (void)kind;
-  return ipt < cap ? ipt : cap;
+  return B_BYTES[n * type_bytes(type) > BT * B_BYTES[0] ? 1 : 0] / type_bytes(type);
 }
 static TuneVal tuned(int kind, int type, int64_t n) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   auto it = g_tune.find(TuneKey{kind, type, bucket_of(n)});
   if (it != g_tune.end()) return it->second;
-  return TuneVal{default_ipt(kind, type, n), BT};
+  // Before tuning, requests of a megabyte and more ask for 512 threads: larger
+  // tiles, so fewer look-backs (0.60 ms against 0.64 for 1000 requests whose
+  // bytes are mostly in such; 36 small ones take 0.017 ms either way).
+  return TuneVal{default_ipt(kind, type, n), n * type_bytes(type) >= (1 << 20) ? 512 : BT};
 }
 // A request's elements per thread in a launch of nt threads: its tuned tile
 // shape where the tuned launch shape is nt, else the same tile size in
@@ -373,7 +541,12 @@ static TuneVal tuned(int kind, int type, int64_t n) {
 static int ipt_for(const acc_request &q, int nt) {
   const TuneVal v = tuned(q.kind, q.type, q.n);
   const int ipt = v.nt == nt ? v.ipt : (int)(((int64_t)v.ipt * v.nt) / nt);
-  return norm_ipt(ipt, q.type, nt);
+  return norm_ipt(ipt, q.type);
+}
+
+// Elements of one item of request q in a launch of nt threads.
+static int64_t item_elems(const acc_request &q, int ipt, int nt) {
+  return (int64_t)ipt * nt * (q.kind == ACC_REQ_FOLD ? B_FOLD_STEPS : 1);
 }
 
 // ---------------------------------------------------------------- plan
@@ -405,9 +578,9 @@ static void *kernel_for(int op, int nt) {
 }
 
 template <int OP> static void launch_op(Batch *b, const BatchArgs &a, cudaStream_t s) {
-  if (b->nt == 128) batch_kernel<OP, 128><<<b->grid, 128, b->smem, s>>>(a);
-  else if (b->nt == 512) batch_kernel<OP, 512><<<b->grid, 512, b->smem, s>>>(a);
-  else batch_kernel<OP, 256><<<b->grid, 256, b->smem, s>>>(a);
+  if (b->nt == 128) batch_kernel<OP, 128><<<b->grid, 160, b->smem, s>>>(a);
+  else if (b->nt == 512) batch_kernel<OP, 512><<<b->grid, 544, b->smem, s>>>(a);
+  else batch_kernel<OP, 256><<<b->grid, 288, b->smem, s>>>(a);
 }
 static int batch_launch_raw(Batch *b, cudaStream_t s) {
   BatchArgs a{b->d_reqs, b->d_item_req, b->nitems, b->d_status, b->d_partials, b->d_req_ticket, b->d_words};
@@ -458,7 +631,6 @@ static int batch_make(int op, const acc_request *reqs, int64_t count, const int3
   std::vector<BReq> h(count);
   std::vector<int32_t> item_req;
   int64_t nitems = 0;
-  size_t max_tile = 0;
   for (int64_t i = 0; i < count; ++i) {
     const acc_request &q = reqs[i];
     if (q.kind != ACC_REQ_FOLD && q.kind != ACC_REQ_SCAN) return ACC_ERR_INVALID;
@@ -466,8 +638,8 @@ static int batch_make(int op, const acc_request *reqs, int64_t count, const int3
     if (q.n < 0 || (q.n > 0 && (!q.in || !q.out))) return ACC_ERR_INVALID;
     if (q.kind == ACC_REQ_FOLD && !q.out) return ACC_ERR_INVALID;  // fold z [] still writes z
     if (q.kind == ACC_REQ_FOLD && q.n == 0 && !q.has_seed) return ACC_ERR_EMPTY;
-    const int ipt = ipt_override ? norm_ipt(ipt_override[i], q.type, nt) : ipt_for(q, nt);
-    const int64_t ts = (int64_t)ipt * nt;
+    const int ipt = ipt_override ? norm_ipt(ipt_override[i], q.type) : ipt_for(q, nt);
+    const int64_t ts = item_elems(q, ipt, nt);
     int64_t ntl = (q.n + ts - 1) / ts;
     if (q.kind == ACC_REQ_FOLD && ntl == 0) ntl = 1;  // fold z [] = z: one (empty) tile writes the seed
     BReq &r = h[i];
@@ -476,8 +648,6 @@ static int batch_make(int op, const acc_request *reqs, int64_t count, const int3
     r.first_item = nitems; r.ntiles = ntl;
     for (int64_t k = 0; k < ntl; ++k) item_req.push_back((int32_t)i);
     nitems += ntl;
-    const size_t tb = (size_t)(ipt + 1) * nt * type_bytes(q.type) + 256;
-    if (tb > max_tile) max_tile = tb;
   }
   if (nitems >= (1ll << 31)) return ACC_ERR_TOO_LARGE;
   Batch *b = new Batch();
@@ -486,7 +656,7 @@ static int batch_make(int op, const acc_request *reqs, int64_t count, const int3
   cudaGetDevice(&b->device);
   b->count = count;
   b->nitems = nitems;
-  b->smem = max_tile < 1024 ? 1024 : max_tile;
+  b->smem = (size_t)(nt / 32) * 2 * b_wbuf_bytes();
   auto fail = [&](cudaError_t e) { batch_free(b); return cuda_status(e); };
   cudaError_t e;
   if ((e = cudaMalloc(&b->d_reqs, sizeof(BReq) * (count ? count : 1))) != cudaSuccess) return fail(e);
@@ -503,7 +673,7 @@ static int batch_make(int op, const acc_request *reqs, int64_t count, const int3
   void *kern = kernel_for(op, nt);
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem);
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt, b->smem) != cudaSuccess || per_sm < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nt + 32, b->smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     per_sm = 1;
   }
@@ -552,12 +722,12 @@ int arena_create(int op, int64_t cap_reqs, int64_t cap_items, BatchArena **out) 
   cudaMemset(b->d_status, 0, sizeof(uint64_t) * 2 * cap_items);
   cudaMemset(b->d_req_ticket, 0, sizeof(uint32_t) * cap_reqs);
   cudaMemset(b->d_words, 0, sizeof(uint32_t) * 64);
-  b->smem = (size_t)B_MAX_TILE_BYTES + BT * 8 + 256;
+  b->smem = (size_t)(BT / 32) * 2 * b_wbuf_bytes();
   b->nt = BT;
   void *kern = kernel_for(op, BT);
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem);
   int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BT, b->smem) != cudaSuccess || per_sm < 1) {
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, BT + 32, b->smem) != cudaSuccess || per_sm < 1) {
     cudaGetLastError();
     per_sm = 1;
   }
@@ -571,7 +741,7 @@ int arena_create(int op, int64_t cap_reqs, int64_t cap_items, BatchArena **out) 
 // Tiles a request will take (0 if it does not fit the batch kernel).
 int64_t arena_tiles(const acc_request &q) {
   const int ipt = ipt_for(q, BT);
-  const int64_t ts = (int64_t)ipt * BT;
+  const int64_t ts = item_elems(q, ipt, BT);
   const int64_t nt = (q.n + ts - 1) / ts;
   return (q.kind == ACC_REQ_FOLD && nt == 0) ? 1 : nt;
 }
@@ -582,7 +752,7 @@ int arena_launch(BatchArena *ar, const acc_request *reqs, int64_t count, cudaStr
   for (int64_t i = 0; i < count; ++i) {
     const acc_request &q = reqs[i];
     const int ipt = ipt_for(q, BT);
-    const int64_t ts = (int64_t)ipt * BT;
+    const int64_t ts = item_elems(q, ipt, BT);
     int64_t nt = (q.n + ts - 1) / ts;
     if (q.kind == ACC_REQ_FOLD && nt == 0) nt = 1;
     if (i >= ar->cap_reqs || nitems + nt > ar->cap_items) return ACC_ERR_TOO_LARGE;
@@ -640,7 +810,8 @@ static int autotune_run(int kind, int type, int bucket, cudaStream_t s, void *bu
   TuneVal pick{default_ipt(kind, type, n), BT};
   // every launch shape, and for each every tile shape
   for (int nt : B_NT) {
-    for (int ipt = 1; ipt <= max_ipt(type, nt); ipt *= 2) {
+    for (int bytes : B_BYTES) {
+      const int ipt = bytes / eb;
       std::vector<int32_t> ov(count, ipt);
       Batch *b = nullptr;
       int st = batch_make(ACC_ADD, reqs.data(), count, ov.data(), nt, &b);
