@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 // into tiles of 256 or 512 rows x 128 B (one 2-D TMA load per 256 rows,
 // 128-byte swizzle, as in the scan; each thread owns one or two adjacent
 // rows), independent of the segment lengths, so every CTA streams the
-// same number of bytes however skewed the segmentation is.  One launch:
+// same number of bytes however skewed the segmentation is:
 //   * a pre-pass (foldseg_tile_index) records for every tile the index of
 //     the first offset at or after its start, so a tile knows its offset
 //     range [kf, ks) from two loads; the CTA copies those offsets
@@ -264,7 +264,12 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 // 88 -> 76 (the index pre-pass is 7 of them).
 constexpr int FT_THREADS = 256;
 constexpr int FT_ROW_BYTES = 128;
-constexpr int FT_CAP = 512;   // tile-relative offsets (and their results) held in shared memory
+// Tile-relative offsets (and their results) held in shared memory: the walk by
+// boundary slots needs all of a tile's, so segments of 11 values (4-byte one-word
+// states: 22) and more on average take it; 768 is what leaves five (three) CTAs
+// per SM.  With 512, 2^26 Int32 values in segments of 30 took 189 us (now 90), 2^26
+// Float32 in segments of 16 179 (130).
+constexpr int FT_CAP = 768;
 // Adjacent 128-byte rows per thread: two for one-word states (a longer walk
 // amortises the per-thread scan and bookkeeping), one for the compensated
 // Float32 pair, whose longer walk code does not pay for itself.
@@ -408,14 +413,15 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
   unsigned char *buf = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t bar;
   __shared__ int64_t s_kf, s_cnt, s_lo, s_hi, s_first_id;
-  __shared__ int s_offs[FT_CAP];
+  __shared__ int16_t s_offs[FT_CAP];  // -1: before the tile (malformed)
+  static_assert(TE < 32768, "16-bit tile-relative offsets");
   __shared__ int s_rowh[FT_THREADS];  // per thread: first offset entry at or after its first value
   __shared__ S s_res[FT_CAP];         // per entry (or, in a slot tile, per boundary): a closed segment's state
   __shared__ S s_wv[NWARP], s_first_v, s_tile_v;
   __shared__ int s_wf[NWARP];
   __shared__ int s_has_first, s_tile_f, s_bad;
   __shared__ uint64_t s_bm[FT_THREADS];  // slot tiles: each thread's boundary positions
-  __shared__ int s_base[FT_THREADS];     // slot tiles: each thread's first boundary slot
+  __shared__ int16_t s_base[FT_THREADS]; // slot tiles: each thread's first boundary slot
   __shared__ int s_nbw[NWARP];
   __shared__ unsigned s_count;           // small: offsets before the tile, and (high half) before its end
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -518,7 +524,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
     const int64_t rel = o - tb;
     if (rel < 0 || (!last_tile && rel >= TE)) bad = true;
     const int r = (int)(rel < 0 ? 0 : (rel > TE ? TE : rel));
-    if (i < FT_CAP) s_offs[i] = (int)(rel < 0 ? -1 : r);
+    if (i < FT_CAP) s_offs[i] = (int16_t)(rel < 0 ? -1 : r);
     int rn = FAR;  // the next entry, or past the tile
     if (k < a.nseg) {
       const int64_t o1 = (int64_t)off[k + 1];
@@ -629,7 +635,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
     for (int w2 = 0; w2 < warp; ++w2) wbase += s_nbw[w2];
     pbase = wbase + incl - nb;
     s_bm[tid] = bm;
-    s_base[tid] = pbase;
+    s_base[tid] = (int16_t)pbase;
     int pk = pbase;
     // fully unrolled: every mask bit is tested at a constant position
     const uint32_t bm_lo = (uint32_t)bm, bm_hi = (uint32_t)(bm >> 32);
