@@ -475,13 +475,25 @@ __global__ void __launch_bounds__(PERM_THREADS, 1) permute_private(PermArgs a) {
   T *out = static_cast<T *>(a.out);
   uint32_t b0 = 0;
   if constexpr (OP == ACC_ADD && std::is_same<T, float>::value) {
-    // four bins per reduction (an untouched bin's -0.0 changes nothing)
+    // four bins per reduction where all four were touched (a reduction may flush
+    // a subnormal target, so an untouched one must not take part)
     if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
+      const uint32_t none = __float_as_uint(idT);
       b0 = m & ~3u;
       for (uint32_t b = 4 * threadIdx.x; b < b0; b += 4 * PERM_THREADS) {
         const float4 v = *reinterpret_cast<const float4 *>(smem_raw + b * sizeof(T));
-        asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
-                     :: "l"(out + b), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+        const float f[4] = {v.x, v.y, v.z, v.w};
+        bool all = true;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) all = all && __float_as_uint(f[k]) != none;
+        if (all) {
+          asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                       :: "l"(out + b), "f"(f[0]), "f"(f[1]), "f"(f[2]), "f"(f[3]) : "memory");
+        } else {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (__float_as_uint(f[k]) != none) atomic_combine<OP, T>(out + b + k, f[k]);
+        }
       }
     }
   }

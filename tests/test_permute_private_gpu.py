@@ -64,3 +64,14 @@ def test_permute_private_out_of_range(acc, dev):
             acc.sync()
         assert e.value.status == 7
         assert out.cpu().tolist() == [1, 60, 0, 1]
+
+
+def test_permute_private_leaves_untouched_bins(acc, dev):
+    # bins that no index names keep their bits: subnormals, negative zero, NaN
+    tiny = torch.tensor([1e-40, -0.0, float("nan"), 1.0, -3e-42, 2.0, 0.0, 5.0, 1e-45], device=dev)
+    idx = torch.tensor([3, 5] * 40, dtype=torch.int32, device=dev)
+    out = acc.permute("+", tiny, idx, torch.ones(80, device=dev))
+    acc.sync()
+    keep = [0, 1, 2, 4, 6, 7, 8]
+    assert torch.equal(out[keep].view(torch.int32), tiny[keep].view(torch.int32))
+    assert out[[3, 5]].tolist() == [41.0, 42.0]
