@@ -229,9 +229,8 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 
 // ----------------------------------------------------------------- tiled single pass
 // 1-D rows with 16-byte aligned values take this path.  The values are cut
-// into tiles of 256 or 512 rows x 128 B (one 2-D TMA load per 256 rows,
-// 128-byte swizzle, as in the scan; each thread owns one or two adjacent
-// rows), independent of the segment lengths, so every CTA streams the
+// into tiles of 256 rows x 128 B (one 2-D TMA load per 128 rows, 128-byte
+// swizzle, as in the scan; each thread owns two adjacent rows), independent of the segment lengths, so every CTA streams the
 // same number of bytes however skewed the segmentation is:
 //   * a pre-pass (foldseg_tile_index) records for every tile the index of
 //     the first offset at or after its start, so a tile knows its offset
@@ -260,23 +259,28 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 // that completed its first segment itself, by a decoupled look-back, held its
 // shared memory for 7,400 cycles of polls and 2,100 of drawing a ticket, of
 // 19,800 (2^22 values); the tiles now wait for no one.  2^26 Float32 values in
-// 2^20 lognormal segments, compensated: 115 -> 100 us, plain 88 -> 75, Int32 max
-// 88 -> 76 (the index pre-pass is 7 of them).
-constexpr int FT_THREADS = 256;
+// 2^20 lognormal segments, compensated: 115 -> 92 us, plain 88 -> 76, Int32 max
+// 88 -> 76 (the index pre-pass is about 5 of them, the completion 3).
+constexpr int FT_THREADS = 128;
 constexpr int FT_ROW_BYTES = 128;
 // Tile-relative offsets (and their results) held in shared memory: the walk by
-// boundary slots needs all of a tile's, so segments of 11 values (4-byte one-word
-// states: 22) and more on average take it; 768 is what leaves five (three) CTAs
-// per SM.  With 512, 2^26 Int32 values in segments of 30 took 189 us (now 90), 2^26
-// Float32 in segments of 16 179 (130).
+// boundary slots needs all of a tile's, so segments of 11 values and more on
+// average take it; 768 is what leaves five CTAs per SM.  With 512, 2^26 Float32
+// values in segments of 16 took 179 us (now 126).
 constexpr int FT_CAP = 768;
-// Adjacent 128-byte rows per thread: two for one-word states (a longer walk
-// amortises the per-thread scan and bookkeeping), one for the compensated
-// Float32 pair, whose longer walk code does not pay for itself.
-template <class S> constexpr int ft_rpt() { return std::is_same<S, F2>::value ? 1 : 2; }
+// Adjacent 128-byte rows per thread: two, so that a thread's share of the tile's
+// bookkeeping and scans (about as much as the walk of one row) is spread over 64
+// 4-byte values, with 128 threads, so that five tiles still fit an SM.  256
+// threads with one row (compensated) or two: 100 us where this takes 92, plain 74
+// (76), 2^26 Int32 values in segments of 16 231 (110: 16,384 values have more
+// boundaries than are kept), 2^25 Float64 140 (116).
+// Over a fused zipWith each tile needs the rows of both arrays: one row each.
+template <bool ZIP> constexpr int ft_rpt() { return ZIP ? 1 : 2; }
 
 struct SegTileArgs {
   const void *in;
+  const void *in2;  // ZIP: the folded element i is zop(in[i], in2[i])
+  int zop;
   const void *off;
   void *out;
   int64_t n, nseg;
@@ -305,20 +309,20 @@ constexpr int TIDX_SHIFT = 35;  // offset indices below 2^35; the epoch above
 // launch: each CTA reads all the offsets (or the lengths, which it scans) into
 // shared memory and finds its tile's first and last offset by counting.
 // 100,003 Int32 values in 1,562 segments by lengths, device time: 23.4 us in
-// three launches (scan of the lengths, index, tiles) -> 13.5; by offsets 17.1
-// -> 13.4.  At the limits, 10^6 Float32 values: 4,000 segments by offsets 14.8 ->
-// 13.8 us, 15,625 segments (three launches) 15.0 -> 13.1.
+// three launches (scan of the lengths, index, tiles) -> 11.1; by offsets 17.0
+// -> 11.1.  At the limits, 10^6 Float32 values: 4,000 segments by offsets 14.8 ->
+// 13.2 us, 15,625 segments (three launches) 15.0 -> 12.1.
 constexpr int FT_SMALL = 4096;
 constexpr int FT_PER = (FT_SMALL + FT_THREADS) / FT_THREADS;  // most offsets per thread
 static_assert(FT_PER % 2 == 1 && FT_PER * FT_THREADS >= FT_SMALL + 1, "an odd number (free of bank conflicts) holds them all");
 
-// Pre-pass: tidx[t] = the first k with off[k] >= t * te (t < ntiles), and
+// Pre-pass: tidx[t] = the first k with off[k] >= t << log_te (t < ntiles), and
 // tidx[ntiles] = nseg + 1, each tagged with the call's epoch so that no
 // clearing is needed.  Thread k writes the tiles whose start lies in
 // (off[k-1], off[k]]; k = nseg + 1 stands for the tiles past the last offset.
 // Decreasing offsets leave tiles unwritten (their stale tag is caught later).
 template <class OT>
-__global__ void foldseg_tile_index(const OT *off, int64_t nseg, int64_t ntiles, int64_t te, uint64_t *tidx,
+__global__ void foldseg_tile_index(const OT *off, int64_t nseg, int64_t ntiles, int log_te, uint64_t *tidx,
                                    uint32_t epoch) {
   const uint64_t tag = (uint64_t)epoch << TIDX_SHIFT;
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k <= nseg + 1;
@@ -327,12 +331,12 @@ __global__ void foldseg_tile_index(const OT *off, int64_t nseg, int64_t ntiles, 
     if (k == 0) t0 = 0;
     else {
       const int64_t lo = (int64_t)off[k - 1];
-      t0 = lo < 0 ? 0 : lo / te + 1;
+      t0 = lo < 0 ? 0 : (lo >> log_te) + 1;
     }
     if (k == nseg + 1) t1 = ntiles - 1;
     else {
       const int64_t hi = (int64_t)off[k];
-      t1 = hi < 0 ? -1 : hi / te;
+      t1 = hi < 0 ? -1 : hi >> log_te;
     }
     if (t1 > ntiles - 1) t1 = ntiles - 1;
     for (int64_t t = t0; t <= t1; ++t) tidx[t] = tag | (uint64_t)k;
@@ -396,12 +400,30 @@ __global__ void __launch_bounds__(256) foldseg_fix(SegTileArgs a) {
   seg_complete<OP, T, PREC>(a, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll);
 }
 
-template <int OP, class T, int PREC, class OT>
-__global__ void __launch_bounds__(FT_THREADS, (ft_rpt<typename Acc<OP, T, PREC>::S>() == 1 ? 5 : 3))
-foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
+// ZIP: a thread zips its own rows of the two arrays' tiles in place before the walk.
+template <class T, int Z>
+__device__ __forceinline__ void seg_zip_row(unsigned char *row, const unsigned char *row2) {
+  constexpr int VEC = 16 / sizeof(T);
+#pragma unroll
+  for (int c = 0; c < FT_ROW_BYTES / 16; ++c) {  // in whatever order: both rows are swizzled alike
+    uint4 v = reinterpret_cast<const uint4 *>(row)[c];
+    const uint4 w = reinterpret_cast<const uint4 *>(row2)[c];
+    T x[VEC], y[VEC];
+    memcpy(x, &v, 16);
+    memcpy(y, &w, 16);
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) x[k] = Prim<Z, T>::ap(x[k], y[k]);
+    memcpy(&v, x, 16);
+    reinterpret_cast<uint4 *>(row)[c] = v;
+  }
+}
+
+template <int OP, class T, int PREC, class OT, bool ZIP = false>
+__global__ void __launch_bounds__(FT_THREADS, ZIP ? 4 : 5)
+foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a, const __grid_constant__ CUtensorMap tin2) {
   using A = Acc<OP, T, PREC>;
   using S = typename A::S;
-  constexpr int FT_RPT = ft_rpt<S>();
+  constexpr int FT_RPT = ft_rpt<ZIP>();
   constexpr int ITEMS = FT_ROW_BYTES / sizeof(T);
   constexpr int VEC = 16 / sizeof(T);
   constexpr int W = FT_RPT * ITEMS;          // values per thread (FT_RPT adjacent rows)
@@ -436,17 +458,18 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
     s_count = 0;
     mbar_init(&bar, 1);
     fence_mbar_init();
-    mbar_expect_tx(&bar, FT_RPT * SUB_BYTES);
+    mbar_expect_tx(&bar, (ZIP ? 2 : 1) * FT_RPT * SUB_BYTES);
 #pragma unroll
     for (int u = 0; u < FT_RPT; ++u)
       tma_load_2d(buf + u * SUB_BYTES, &tin, 0, (int)((tile * FT_RPT + u) * FT_THREADS), &bar);
+    if constexpr (ZIP) tma_load_2d(buf + SUB_BYTES, &tin2, 0, (int)(tile * FT_THREADS), &bar);
   }
   __syncthreads();
   const int64_t tb = tile * TE;
   const bool last_tile = tile == a.ntiles - 1;
   if (a.small) {
     const OT *given = off;
-    OT *all = reinterpret_cast<OT *>(buf + FT_RPT * SUB_BYTES);
+    OT *all = reinterpret_cast<OT *>(buf + (ZIP ? 2 : 1) * FT_RPT * SUB_BYTES);
     const int no = (int)a.nseg + 1, ng = a.small == 2 ? no - 1 : no;
     const int per = ((no + FT_THREADS - 1) / FT_THREADS) | 1;  // consecutive offsets per thread, an odd number
     {
@@ -581,14 +604,27 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
     finish(0, 0, -1, true);
     return;
   }
+  if constexpr (ZIP) {
+    unsigned char *row = buf + tid * FT_ROW_BYTES;
+    const unsigned char *row2 = row + SUB_BYTES;
+    switch (a.zop) {
+      case ACC_ADD: seg_zip_row<T, ACC_ADD>(row, row2); break;
+      case ACC_MUL: seg_zip_row<T, ACC_MUL>(row, row2); break;
+      case ACC_MIN: seg_zip_row<T, ACC_MIN>(row, row2); break;
+      default: seg_zip_row<T, ACC_MAX>(row, row2); break;
+    }
+  }
   // The values after the last whole row (TMA left zeros there; the positions
   // past the last value are masked below).
   if (a.full_rows >= tile * (FT_RPT * FT_THREADS) && a.full_rows < (tile + 1) * (FT_RPT * FT_THREADS)) {
+    if constexpr (ZIP) __syncthreads();  // after its owner has zipped that row's zeros
     const int64_t gi = a.full_rows * ITEMS + tid;
     if (tid < ITEMS && gi < a.n) {
       const int r = (int)(a.full_rows - tile * (FT_RPT * FT_THREADS)), rr = r % FT_THREADS;
+      T v = static_cast<const T *>(a.in)[gi];
+      if constexpr (ZIP) v = zip_elem(a.zop, v, static_cast<const T *>(a.in2)[gi]);
       *reinterpret_cast<T *>(buf + (r / FT_THREADS) * SUB_BYTES + rr * FT_ROW_BYTES + (((tid / VEC) ^ (rr & 7)) << 4) +
-                             (tid % VEC) * sizeof(T)) = static_cast<const T *>(a.in)[gi];
+                             (tid % VEC) * sizeof(T)) = v;
     }
     __syncthreads();
   }
@@ -825,33 +861,39 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a) {
 
 // One launcher per kernel instantiation, so that each gets its own
 // shared-memory attribute (the tile needs more than the default 48 KB).
-template <int OP, class T, int PREC, class OT>
-int launch_foldseg_tile(const CUtensorMap &tin, const SegTileArgs &a, int64_t ntiles, cudaStream_t s) {
-  constexpr int FT_RPT = ft_rpt<typename Acc<OP, T, PREC>::S>();
-  const size_t tile = (size_t)FT_RPT * FT_THREADS * FT_ROW_BYTES + 1024;
+template <int OP, class T, int PREC, class OT, bool ZIP>
+int launch_foldseg_tile(const CUtensorMap &tin, const SegTileArgs &a, int64_t ntiles, cudaStream_t s,
+                        const CUtensorMap &tin2) {
+  constexpr int FT_RPT = ft_rpt<ZIP>();
+  const size_t tile = (size_t)(ZIP ? 2 : 1) * FT_RPT * FT_THREADS * FT_ROW_BYTES + 1024;
   const size_t all = (size_t)(FT_PER * FT_THREADS + FT_THREADS / 32) * sizeof(OT);  // small: the offsets, the warps' sums
   const size_t smem = tile + (a.small ? all : 0);
-  auto kern = foldseg_tile_kernel<OP, T, PREC, OT>;
+  auto kern = foldseg_tile_kernel<OP, T, PREC, OT, ZIP>;
   static std::atomic<uint64_t> attr_done{0};
   smem_attrs_once(kern, (int)(tile + all), attr_done);
-  kern<<<(unsigned)ntiles, FT_THREADS, smem, s>>>(tin, a);
+  kern<<<(unsigned)ntiles, FT_THREADS, smem, s>>>(tin, a, tin2);
   const int st = check_launch();
   if (st || a.small) return st;
   foldseg_fix<OP, T, PREC><<<(unsigned)cdiv_h(ntiles, 256), 256, 0, s>>>(a);
   return check_launch();
 }
 
-template <int OP, class T, int PREC>
+template <int OP, class T, int PREC, bool ZIP = false>
 int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bool lengths, T *out, int64_t inner,
-                       int64_t nseg, bool has_seed, uint64_t seed, cudaStream_t s, bool *taken) {
+                       int64_t nseg, bool has_seed, uint64_t seed, cudaStream_t s, bool *taken,
+                       const T *in2 = nullptr, int zop = 0) {
   constexpr int ITEMS = FT_ROW_BYTES / sizeof(T);
-  constexpr int FT_RPT = ft_rpt<typename Acc<OP, T, PREC>::S>();
+  constexpr int FT_RPT = ft_rpt<ZIP>();
   constexpr int64_t TE = (int64_t)FT_THREADS * FT_RPT * ITEMS;
+  constexpr int LOG_TE = 31 - __builtin_clz((unsigned)TE);
+  static_assert(TE == int64_t(1) << LOG_TE, "tiles of a power of two values");
   *taken = false;
   const int64_t full_rows = inner / ITEMS;
-  CUtensorMap tin;
+  CUtensorMap tin, tin2;
   memset(&tin, 0, sizeof(tin));
-  if (full_rows == 0 || !encode_2d(&tin, in, sizeof(T), ITEMS, full_rows, FT_ROW_BYTES, ITEMS, FT_THREADS, true))
+  memset(&tin2, 0, sizeof(tin2));
+  if (full_rows == 0 || !encode_2d(&tin, in, sizeof(T), ITEMS, full_rows, FT_ROW_BYTES, ITEMS, FT_THREADS, true) ||
+      (ZIP && !encode_2d(&tin2, in2, sizeof(T), ITEMS, full_rows, FT_ROW_BYTES, ITEMS, FT_THREADS, true)))
     return ACC_OK;  // not describable by TMA: the caller uses the per-segment kernels
   // One tile more than the values need when they fill the last tile exactly:
   // that tile holds the boundary at position n.
@@ -860,6 +902,11 @@ int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bo
   if (nseg + 2 >= (1ll << TIDX_SHIFT)) return ACC_OK;
   const bool small = nseg <= FT_SMALL && ntiles <= 2 * (int64_t)device_info().sms;
   if (lengths && !small) return ACC_OK;  // the caller scans the lengths first
+  // Over a zipWith, two arrays' tiles leave too few CTAs per SM for long calls:
+  // 67,860 Float32 values 41 -> 16 us, 10^6 28 -> 23, 2^25 115 -> 155.  Float64
+  // states are bound by their additions there too (2^24 Float64 212 -> 166).
+  if (ZIP && ntiles > 2 * (int64_t)device_info().sms && !std::is_same<typename Acc<OP, T, PREC>::S, double>::value)
+    return ACC_OK;
   *taken = true;
   const size_t slot_bytes = (size_t)ntiles * sizeof(SegSlot);
   int st = ws_scratch(w, slot_bytes + (size_t)(ntiles + 1) * sizeof(uint64_t));
@@ -867,6 +914,7 @@ int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bo
   uint64_t *tidx = reinterpret_cast<uint64_t *>(static_cast<char *>(w->scratch) + slot_bytes);
   SegTileArgs a{};
   a.in = in; a.off = off; a.out = out;
+  a.in2 = in2; a.zop = zop;
   a.n = inner; a.nseg = nseg;
   a.full_rows = full_rows; a.ntiles = ntiles;
   a.seed = seed; a.has_seed = has_seed;
@@ -881,16 +929,16 @@ int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bo
     int64_t pb = cdiv_h(nseg + 2, 256);
     if (pb > (int64_t)d.sms * 8) pb = (int64_t)d.sms * 8;
     if (off64)
-      foldseg_tile_index<int64_t><<<(unsigned)pb, 256, 0, s>>>(static_cast<const int64_t *>(off), nseg, ntiles, TE,
+      foldseg_tile_index<int64_t><<<(unsigned)pb, 256, 0, s>>>(static_cast<const int64_t *>(off), nseg, ntiles, LOG_TE,
                                                                 tidx, a.epoch);
     else
-      foldseg_tile_index<int32_t><<<(unsigned)pb, 256, 0, s>>>(static_cast<const int32_t *>(off), nseg, ntiles, TE,
+      foldseg_tile_index<int32_t><<<(unsigned)pb, 256, 0, s>>>(static_cast<const int32_t *>(off), nseg, ntiles, LOG_TE,
                                                                 tidx, a.epoch);
     st = check_launch();
     if (st) return st;
   }
-  return off64 ? launch_foldseg_tile<OP, T, PREC, int64_t>(tin, a, ntiles, s)
-               : launch_foldseg_tile<OP, T, PREC, int32_t>(tin, a, ntiles, s);
+  return off64 ? launch_foldseg_tile<OP, T, PREC, int64_t, ZIP>(tin, a, ntiles, s, tin2)
+               : launch_foldseg_tile<OP, T, PREC, int32_t, ZIP>(tin, a, ntiles, s, tin2);
 }
 
 // ----------------------------------------------------------------- host side
@@ -935,6 +983,11 @@ int foldseg_typed(Workspace *w, const T *in, const void *off, int off64, T *out,
   return check_launch();
 }
 
+static bool foldseg_per_segment() {
+  static const bool v = getenv("ACC_GB300_FOLDSEG") && strcmp(getenv("ACC_GB300_FOLDSEG"), "segments") == 0;
+  return v;
+}
+
 // `lengths`: `off` holds the segments' lengths; *taken says whether the call
 // was made (one launch scans them too), and nothing else is tried.
 int foldseg_dispatch(Workspace *w, int op, int type, int prec, const void *in, const void *off,
@@ -949,8 +1002,7 @@ int foldseg_dispatch(Workspace *w, int op, int type, int prec, const void *in, c
         constexpr int P = decltype(pc)::value;
         // Rows of one segmented vector take the tiled single pass unless
         // ACC_GB300_FOLDSEG=segments asks for the per-segment kernels.
-        static const bool per_segment =
-            getenv("ACC_GB300_FOLDSEG") && strcmp(getenv("ACC_GB300_FOLDSEG"), "segments") == 0;
+        const bool per_segment = foldseg_per_segment();
         if (outer == 1 && !per_segment) {
           bool taken = false;
           const int st = foldseg_tile_typed<OP, T, P>(w, static_cast<const T *>(in), off, off64, lengths,
@@ -1011,11 +1063,11 @@ extern "C" int acc_fold_seg_lengths(int op, int type, int prec, const void *in, 
   // The offsets live at the END of the scratch area.  The front part,
   // list_bytes, holds what the fold itself keeps in scratch: the per-segment
   // path's long-segment list (at most inner / LONG_SEG + 1 entries) or the
-  // tiled path's slots and tile index (40 bytes per tile of at least 8192
+  // tiled path's slots and tile index (40 bytes per tile of at least 4096
   // values), both within list_bytes, so neither grows (and moves) the
   // scratch under the offsets.
   const size_t esz = length_type == ACC_I64 ? 8 : 4;
-  const size_t list_bytes = (size_t)(inner / LONG_SEG + 2) * 2 * sizeof(int64_t) + 512;
+  const size_t list_bytes = (size_t)(inner / LONG_SEG + 2) * 3 * sizeof(int64_t) + 512;
   const size_t off_bytes = (size_t)(nseg + 1) * esz;
   st = ws_scratch(w, list_bytes + off_bytes + 256);
   if (st) return st;
@@ -1027,8 +1079,10 @@ extern "C" int acc_fold_seg_lengths(int op, int type, int prec, const void *in, 
 
 // foldSeg f z (zipWith g xs ys): the reference fuses the producer into the
 // segmented fold's kernel (its delayed input, PTX/CodeGen/FoldSeg.hs:56-458
-// reading a MIRDelayed array).  Here the per-segment kernels read both arrays
-// and zip each element as they load it (the zipped array is never written).
+// reading a MIRDelayed array).  Here the tiles of both arrays are zipped in
+// shared memory before the walk (short 1-D calls, both 16-byte aligned), or the
+// per-segment kernels zip each element as they load it; the zipped array is never
+// written.
 // f in {+, min, max}, g in {+, *, min, max}, Int32 / Int64 / Float32 /
 // Float64, as for the fused fold and scans.
 extern "C" int acc_fold_seg_zipwith(int op, int zop, int type, int prec, const void *xs, const void *ys,
@@ -1056,6 +1110,13 @@ extern "C" int acc_fold_seg_zipwith(int op, int zop, int type, int prec, const v
       } else {
         return with_prec<OP, T>(prec, [&](auto pc) -> int {
           constexpr int P = decltype(pc)::value;
+          if (outer == 1 && !foldseg_per_segment()) {
+            bool taken = false;
+            const int st2 = foldseg_tile_typed<OP, T, P, true>(
+                w, static_cast<const T *>(xs), offsets, offset_type == ACC_I64, false, static_cast<T *>(out), inner, nseg,
+                seed != nullptr, sb, s, &taken, static_cast<const T *>(ys), zop);
+            if (taken || st2) return st2;
+          }
           return foldseg_typed<OP, T, P, true>(w, static_cast<const T *>(xs), offsets, offset_type == ACC_I64,
                                                static_cast<T *>(out), outer, inner, nseg, seed != nullptr, sb, s,
                                                static_cast<const T *>(ys), zop);

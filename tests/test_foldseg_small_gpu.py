@@ -68,3 +68,27 @@ def test_scan_rows_chunks(acc, orc, dev, t, op, flavour):
     for shape in ((1,), (32 * per - 1,), (32 * per + 1,), (1024 * per,), (1024 * per + 1,), (3, 1024 * per + 1), (5, 33 * per),
                   (2, 3 * 1024 * per + 7), (700, 31)):
         run_scan(acc, orc, dev, t, op, shape, d, k)
+
+
+@pytest.mark.parametrize("t,op", [("f32", "+"), ("i32", "max"), ("i64", "+"), ("f64", "min")])
+@pytest.mark.parametrize("zop", ["+", "*", "min", "max"])
+@pytest.mark.parametrize("nseg,n,off_a,off_b", [(1, 40, 0, 0), (700, 8192 * 3, 0, 0), (5000, 300_007, 0, 0), (9, 8192 * 700 + 33, 0, 0),
+                                                (500, 30_001, 0, 1), (500, 30_001, 1, 1)])
+def test_foldseg_zip_tiles(acc, orc, dev, t, op, zop, nseg, n, off_a, off_b):
+    # the fused zipWith on the tiled form (both arrays 16-byte aligned) and beside it
+    rng = case_rng("ziptiles", t, op, zop, nseg, n, off_a, off_b)
+    dt = TYPES[t]
+    x, y = gen(dt, "+", n + off_a, rng), gen(dt, "+", n + off_b, rng)
+    off = np.concatenate([[0], np.cumsum(lengths_of("cut" if nseg > 1 else "one", nseg, n, rng))]).astype(np.int32)
+    z = {"+": 0, "max": np.iinfo(np.int32).min, "min": 7.0}[op]
+    got = acc.fold_seg_zipwith(op, zop, z, torch.from_numpy(x).to(dev)[off_a:], torch.from_numpy(y).to(dev)[off_b:],
+                               torch.from_numpy(off).to(dev))
+    acc.sync()
+    with np.errstate(over="ignore"):
+        v = {"+": np.add, "*": np.multiply, "min": np.minimum, "max": np.maximum}[zop](x[off_a:], y[off_b:])
+    ref = orc.fold_seg(op, z, v, off)
+    ref64 = ab = None
+    if np.dtype(dt).kind == "f":
+        ref64 = orc.fold_seg(op, z, v.astype(np.float64), off)
+        ab = orc.fold_seg("+", 0, np.abs(v.astype(np.float64)), off)
+    assert_fold_close(got.cpu().numpy(), ref, ref64, ab, dt, op)
