@@ -183,6 +183,15 @@ template <> struct Acc<ACC_ADD, float, PREC_F64> {
   __device__ __forceinline__ static float lower(S a) { return __double2float_rn(a); }
 };
 
+// Whether a row may be combined one value after the other where a tree was
+// taken before: the result does not depend on the order (integers, max, min), or
+// carries its rounding errors along (Float32 (+) compensated or in FP64).  A
+// plain floating-point sum of a long row loses less in a tree.
+template <int OP, class T, int PREC> constexpr bool serial_exact() {
+  return (T)0.5 == (T)0 || OP == ACC_MAX || OP == ACC_MIN ||
+         (OP == ACC_ADD && sizeof(T) == 4 && PREC != PREC_PLAIN);
+}
+
 // ----------------------------------------------------------------- bit casts
 template <class S> __device__ __forceinline__ uint64_t to_bits(S v) {
   static_assert(sizeof(S) <= 8, "state too large");

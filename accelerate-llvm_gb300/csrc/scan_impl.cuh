@@ -1284,9 +1284,107 @@ __global__ void __launch_bounds__(256) scan_rows_warp_kernel(RowScanArgs a) {
   }
 }
 
+// Rows of at most 512 bytes, many of them: one lane per row.  A warp loads 32
+// rows (consecutive in memory) coalesced into shared memory, each lane scans its
+// row there, and the results leave coalesced; no shuffles, and no lane idles on
+// a short row.  Rows are kept at an odd pitch, free of bank conflicts, with the
+// extra slot of scanl z / scanr z.
+// Bound: HBM for rows of up to about 32 values, the loads that the shared memory
+// leaves room for (33 KB per CTA at 512 bytes) beyond.  2^26 Float32 in rows of
+// 16, scanl1: a warp per row 738 us, here 102 (5.3 TB/s); Int32 504 -> 87; 2^26
+// Int64 in rows of 24, scanl 490 -> 176 (6.2 TB/s).
+constexpr int LANE_BYTES = 512;
+constexpr int LANE_WARPS = 2, LANE_U = 8;
+
+template <int OP, class T, int PREC, bool R2L, bool ZIP = false, bool MAP = false>
+__global__ void __launch_bounds__(LANE_WARPS * 32) scan_rows_lane_kernel(RowScanArgs a, uint32_t inv_in, uint32_t inv_out) {
+  using A = Acc<OP, T, PREC>;
+  using S = typename A::S;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int lane = threadIdx.x & 31;
+  const int inner = (int)a.inner, outer_pitch = (int)a.out_pitch, pitch = (inner + 1) | 1;
+  T *buf = reinterpret_cast<T *>(smem_raw) + (threadIdx.x >> 5) * (32 * pitch);
+  T *row = buf + lane * pitch;
+  const T mapc = from_bits<T>(a.mapc);
+  (void)mapc;
+  const int64_t warps = (int64_t)gridDim.x * LANE_WARPS;
+  for (int64_t r0 = ((int64_t)blockIdx.x * LANE_WARPS + (threadIdx.x >> 5)) * 32; r0 < a.outer; r0 += warps * 32) {
+    const int rows = a.outer - r0 < 32 ? (int)(a.outer - r0) : 32;
+    const T *src = static_cast<const T *>(a.in) + r0 * inner;
+    const T *src2 = ZIP ? static_cast<const T *>(a.in2) + r0 * inner : nullptr;
+    (void)src2;
+    // element e of the 32 rows is of row e / inner, kept at its pitch
+    // (inv_in: ceil(2^32 / inner), exact here); eight loads in flight, the last ones too
+    const int total_in = rows * inner;
+    for (int e0 = lane; e0 < total_in; e0 += LANE_U * 32) {
+      T x[LANE_U], y[ZIP ? LANE_U : 1];
+#pragma unroll
+      for (int u = 0; u < LANE_U; ++u) {
+        const int e = e0 + u * 32;
+        x[u] = e < total_in ? src[e] : T(0);
+        if constexpr (ZIP) y[u] = e < total_in ? src2[e] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < LANE_U; ++u) {
+        const int e = e0 + u * 32;
+        if constexpr (ZIP) x[u] = zip_elem(a.zop, x[u], y[u]);
+        else if constexpr (MAP) x[u] = zip_elem(a.zop, x[u], mapc);
+        if (e < total_in) buf[e + (int)__umulhi((uint32_t)e, inv_in) * (pitch - inner)] = x[u];
+      }
+    }
+    __syncwarp();
+    S run = a.has_seed ? A::lift(from_bits<T>(a.seed)) : A::id();
+#pragma unroll 4
+    for (int jj = 0; jj < inner; ++jj) {
+      const int j = R2L ? inner - 1 - jj : jj;
+      const T x = row[j];
+      T y;
+      if (a.exclusive) { y = A::lower(run); run = A::push(run, x); }
+      else { run = A::push(run, x); y = A::lower(run); }
+      row[j] = y;
+    }
+    const T total = A::lower(run);
+    if (a.sums && lane < rows) static_cast<T *>(a.sums)[r0 + lane] = total;
+    row[inner] = a.seed_at_end ? from_bits<T>(a.seed) : total;  // the extra slot, where there is one
+    __syncwarp();
+    T *dst = static_cast<T *>(a.out) + r0 * outer_pitch;
+    const int total_out = rows * outer_pitch;
+    for (int o0 = lane; o0 < total_out; o0 += LANE_U * 32)
+#pragma unroll
+      for (int u = 0; u < LANE_U; ++u) {
+        const int o = o0 + u * 32;
+        if (o < total_out) dst[o] = buf[o + (int)__umulhi((uint32_t)o, inv_out) * (pitch - outer_pitch)];
+      }
+    __syncwarp();
+  }
+}
+
+// The lane form's range.  512 bytes: scanl over 2^26 Int32 in rows of 128 386 -> 190 us, a
+// fused zipWith 257 -> 171.  From 32 rows per SM on: 5000 rows of 32 take 10.3 us with
+// a CTA per row, 4.2 here.  Where a warp per row is the other form, from 512 rows
+// per value of a row on: a lane walks its row alone, and 16,384 rows of 64 take
+// 5.0 us by warps, 6.4 by lanes (32,768 rows of 32: 5.8 and 4.6).  The sums that
+// lose less in a tree stay with the shuffles.
+template <int OP, class T, int PREC> bool rows_lane(int64_t outer, int64_t inner) {
+  const int64_t sms = device_info().sms;
+  return serial_exact<OP, T, PREC>() && inner > 1 && inner * (int64_t)sizeof(T) <= LANE_BYTES &&
+         outer >= sms * 32 && (outer < sms * 64 || outer >= inner * 512);
+}
+
 template <int OP, class T, int PREC, bool R2L, bool ZIP = false, bool MAP = false>
 int launch_scan_rows(const RowScanArgs &a, cudaStream_t s) {
   const Device &d = device_info();
+  if constexpr (serial_exact<OP, T, PREC>()) {
+    if (rows_lane<OP, T, PREC>(a.outer, a.inner)) {
+      const size_t smem = (size_t)LANE_WARPS * 32 * (((size_t)a.inner + 1) | 1) * sizeof(T);
+      int64_t blocks = cdiv_h(a.outer, 32 * LANE_WARPS);
+      if (blocks > (int64_t)d.sms * 32) blocks = (int64_t)d.sms * 32;
+      auto inv = [](int64_t n) { return (uint32_t)(((1ull << 32) + n - 1) / n); };
+      scan_rows_lane_kernel<OP, T, PREC, R2L, ZIP, MAP><<<(unsigned)blocks, LANE_WARPS * 32, smem, s>>>(
+          a, inv(a.inner), inv(a.out_pitch));
+      return check_launch();
+    }
+  }
   if (a.inner <= 512 && a.outer >= (int64_t)d.sms * 64) {
     // a warp per row: 8 rows per CTA
     int64_t blocks = cdiv_h(a.outer, 8);
@@ -1461,8 +1559,13 @@ int scan_typed(Workspace *w, int dir, int kind, const T *in, T *out, T *sums, in
   }
   if constexpr (!ZIP && !MAP) {
     // Long scanl1 / scanr1 / scanl' / scanr' over rows: one segmented pass
-    // over the whole array (at least four 32 KiB tiles per SM).
-    if (outer * inner * (int64_t)sizeof(T) >= (int64_t)device_info().sms * 4 * L2S_TILE) {
+    // over the whole array (at least four 32 KiB tiles per SM).  Short rows
+    // of inner + 1 results are quicker by lanes (2^26 Int32 in rows of 48:
+    // scanl 405 -> 100 us, scanl' 127 -> 100, but at 64 scanr' 115 -> 122 and
+    // scanl1 at 24..64 is as fast in the pass).
+    if (outer * inner * (int64_t)sizeof(T) >= (int64_t)device_info().sms * 4 * L2S_TILE &&
+        !(kind == ACC_SCAN_SEEDED && rows_lane<OP, T, PREC>(outer, inner)) &&
+        !(kind == ACC_SCAN_PRIME && inner * (int64_t)sizeof(T) < 256 && rows_lane<OP, T, PREC>(outer, inner))) {
       bool launched = false;
       const int pc = PREC == 1 ? ACC_PREC_COMPENSATED : (PREC == 2 ? ACC_PREC_FP64ACC : ACC_PREC_PLAIN);
       const int st = scan_rows_seg(w, OP, type_code<T>(), pc, r2l, kind, in, out, kind == ACC_SCAN_PRIME ? sums : nullptr,
