@@ -230,6 +230,21 @@ template <class S> __device__ __forceinline__ S shfl_up(S v, int d) {
     return from_bits<S>(((uint64_t)hi << 32) | lo);
   }
 }
+template <class S> __device__ __forceinline__ S shfl_xor(S v, int m) {
+  if constexpr (sizeof(S) == 4) {
+    uint32_t b;
+    memcpy(&b, &v, 4);
+    b = __shfl_xor_sync(0xffffffffu, b, m);
+    memcpy(&v, &b, 4);
+  } else {
+    const uint64_t b = to_bits(v);
+    const uint32_t lo = __shfl_xor_sync(0xffffffffu, (uint32_t)b, m);
+    const uint32_t hi = __shfl_xor_sync(0xffffffffu, (uint32_t)(b >> 32), m);
+    const uint64_t r = ((uint64_t)hi << 32) | lo;
+    memcpy(&v, &r, sizeof(S));
+  }
+  return v;
+}
 template <class S> __device__ __forceinline__ S shfl_idx(S v, int src) {
   if constexpr (sizeof(S) == 4) {
     uint32_t b; memcpy(&b, &v, 4);

@@ -9,6 +9,8 @@
 //   * fold_rows_lane    -- rows of 6 to 72 values, many of them: one lane per
 //                          row, through shared memory;
 //   * fold_rows_thread  -- inner <= 16: one thread per row;
+//   * fold_rows_multi   -- rows of 17 to 96 values (8-byte types: 200), many of
+//                          them: eight rows per warp at a time;
 //   * fold_rows_warp    -- short rows, many of them: one warp per row;
 //   * fold_split        -- long rows: a row is cut over G CTAs, each thread
 //                          streams 16-byte vectors (4 in flight), the CTA
@@ -224,6 +226,72 @@ __global__ void __launch_bounds__(FOLD_LANE_WARPS * 32) fold_rows_lane(FoldArgs 
   }
 }
 
+// Rows of 17 to 96 values (8-byte types: up to 200), many of them: a warp folds 8 rows at a time.  One row
+// leaves most of a warp's load slots empty and pays five shuffle steps; here 8
+// rows' loads (128 or 256 bytes each) are in flight together, and the lanes' sums of
+// the 8 rows are turned while they are combined: 4 + 2 + 1 exchanges bring every
+// lane down to one row's sum, two more finish it, 9 instead of 40.
+// Bound: HBM, for Float64 the FP64 pipe.  2^26 values against one row at a time:
+// Float32 plain in rows of 24 424 -> 70 us, of 64 165 -> 80, compensated in rows of 80
+// 177 -> 140; Int32 of 96 120 -> 67; Int64 of 64 195 -> 88 (6.1 TB/s), of 96 136 -> 81;
+// Float64 of 64 875 -> 212, of 200 449 -> 174.
+// The range: beyond it a row fills a warp's 16-byte loads and these narrower ones
+// are slower (Int32 of 200 61 us and 80 here; compensated Float32 of 128 113 and 159;
+// Int64 of 64 with a fused zipWith 240 and 254, of 160 177 and 222; Float64, which
+// waits for its additions, gains up to 200).  From 64 rows per SM on: fewer leave
+// warps idle that one row each would use.
+constexpr int FOLD_MULTI_R = 8;
+template <class T, int ZOP> constexpr int64_t fold_multi_max() {
+  return sizeof(T) == 4 ? 96 : (T)0.5 != (T)0 ? 200 : zips<ZOP>() ? 63 : 112;
+}
+
+template <int OP, class T, int PREC, int ZOP = NO_ZIP>
+__global__ void __launch_bounds__(256) fold_rows_multi(FoldArgs a) {
+  using A = Acc<OP, T, PREC>;
+  using S = typename A::S;
+  const int lane = threadIdx.x & 31, inner = (int)a.inner;
+  const T c = from_bits<T>(a.mapc);
+  const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  for (int64_t r0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * FOLD_MULTI_R; r0 < a.outer;
+       r0 += warps * FOLD_MULTI_R) {
+    const int rows = a.outer - r0 < FOLD_MULTI_R ? (int)(a.outer - r0) : FOLD_MULTI_R;
+    const T *p = static_cast<const T *>(a.in) + r0 * inner;
+    const T *q = zips<ZOP>() ? static_cast<const T *>(a.in2) + r0 * inner : nullptr;
+    S acc[FOLD_MULTI_R];
+#pragma unroll
+    for (int r = 0; r < FOLD_MULTI_R; ++r) acc[r] = A::id();
+    auto step = [&](int k) {
+      T x[FOLD_MULTI_R];
+#pragma unroll
+      for (int r = 0; r < FOLD_MULTI_R; ++r) x[r] = zip_at<ZOP, T>(p, q, (r < rows ? r : 0) * inner + k, c);
+#pragma unroll
+      for (int r = 0; r < FOLD_MULTI_R; ++r) acc[r] = A::push(acc[r], x[r]);
+    };
+    int k = lane;  // whole steps of 32 first: every lane takes the same number
+#pragma unroll 2
+    for (int k0 = 32; k0 <= inner; k0 += 32, k += 32) step(k);
+    if (k < inner) step(k);
+    __syncwarp();
+#pragma unroll
+    for (int w = FOLD_MULTI_R / 2; w >= 1; w >>= 1) {  // lane bit 4, 3, 2 chooses the rows that it keeps
+      const bool up = lane & (w * 4);
+#pragma unroll
+      for (int i = 0; i < w; ++i) {
+        const S keep = up ? acc[i + w] : acc[i];
+        const S send = up ? acc[i] : acc[i + w];
+        acc[i] = A::comb(keep, shfl_xor(send, w * 4));
+      }
+    }
+    acc[0] = A::comb(acc[0], shfl_xor(acc[0], 2));
+    acc[0] = A::comb(acc[0], shfl_xor(acc[0], 1));
+    const int r = lane >> 2;
+    if ((lane & 3) == 0 && r < rows) {
+      if (a.has_seed) acc[0] = A::comb(A::lift(from_bits<T>(a.seed)), acc[0]);
+      static_cast<T *>(a.out)[r0 + r] = A::lower(acc[0]);
+    }
+  }
+}
+
 struct SplitArgs {
   const void *in;
   void *out;
@@ -300,6 +368,12 @@ int fold_typed(Workspace *w, const T *in, T *out, int64_t outer, int64_t inner, 
     int64_t blocks = cdiv_h(outer, 256);
     if (blocks > (int64_t)d.sms * 16) blocks = (int64_t)d.sms * 16;
     fold_rows_thread<OP, T, PREC, ZOP><<<(unsigned)blocks, 256, 0, s>>>(fa);
+    return check_launch();
+  }
+  if (inner <= fold_multi_max<T, ZOP>() && outer >= (int64_t)d.sms * FOLD_MULTI_R * 8) {
+    int64_t blocks = cdiv_h(outer, 8 * FOLD_MULTI_R);
+    if (blocks > (int64_t)d.sms * 32) blocks = (int64_t)d.sms * 32;
+    fold_rows_multi<OP, T, PREC, ZOP><<<(unsigned)blocks, 256, 0, s>>>(fa);
     return check_launch();
   }
   const int64_t row_bytes = inner * (int64_t)sizeof(T);

@@ -41,3 +41,16 @@ def test_rows_lane_large(acc, orc, dev, t, op, shape):
     # above the size of the segmented pass, which the short rows of scanl / scanr and of scanl' / scanr' leave
     for d, k in FLAVOURS:
         run_scan(acc, orc, dev, t, op, shape, d, k)
+
+
+@pytest.mark.parametrize("t,op", [("i32", "+"), ("f32", "*"), ("f32", "+"), ("i64", "min"), ("f64", "+"), ("f64", "max")])
+@pytest.mark.parametrize("shape", [(9728, 17), (9735, 31), (9736, 32), (9727, 33), (9729, 64), (9730, 96), (9731, 97), (9732, 112),
+                                   (9733, 113), (9734, 200), (9735, 201), (77_827, 80)])
+def test_rows_by_eights(acc, orc, dev, t, op, shape):
+    # a warp folds eight rows at a time: whole and partial steps of 32 values, one to eight rows in the last warp
+    for prec in ("default", "plain") if (t, op) == ("f32", "+") else (None,):
+        run_fold(acc, orc, dev, t, op, shape, seeded=True, prec=prec)
+    run_fold(acc, orc, dev, t, op, shape, seeded=False, offset=1)
+    if op == "+":
+        run_zip(acc, orc, dev, t, "+", "*", shape, True, offset=1)
+        run_fold_map(acc, orc, dev, t, "+", "*", shape, True)
