@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 // end of the row.  Three launches: the index pre-pass, the tiles and the
 // completion; one for short calls.  Offsets that decrease or leave [0, n] raise
 // ACC_ERR_INDEX; the tile then writes nothing.
-// Bound: issue (about 38 thread instructions per value, compensated).  A tile
+// Bound: issue (about 30 thread instructions per value, compensated).  A tile
 // that completed its first segment itself, by a decoupled look-back, held its
 // shared memory for 7,400 cycles of polls and 2,100 of drawing a ticket, of
 // 19,800 (2^22 values); the tiles now wait for no one.  2^26 Float32 values in

@@ -48,13 +48,13 @@ BYTES = {
 # DRAM bytes per full-size launch of each skeleton's kernel:
 # dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the
 # `bench.py --only <skeleton> --scale <s>` small case, scaled by the units
-# processed to the full launch (traffic grows in proportion; the stencil case
-# is already full size).  Summaries with the commands sit in profiles/.
+# processed to the full launch (traffic grows in proportion; permute and stencil
+# are captures of the full launch).  Summaries with the commands sit in profiles/.
 NCU_TRAFFIC = {
     "scan": int((270.588416e6 + 207.724288e6) * 8),   # 2^25 Int64 -> 2^28 (scan_l2_kernel)
     "fold": int((268.478208e6 + 2.757376e6) * 4),     # 2^26 Float32 -> 2^28
-    "permute": int((268.722688e6 + 2.906368e6) * 4),  # 2^26 indices -> 2^28
-    "stencil": int(292.122624e6 + 222.595328e6),      # 8192^2, full size
+    "permute": int(1074.075392e6 + 2.847744e6),       # 2^28 indices, full size (permute_count16)
+    "stencil": int(269.182976e6 + 214.3168e6),        # 8192^2, full size (stencil_rows_kernel)
 }
 
 # foldSeg workload: 2^26 Float32 values ~ N(0,1) in 2^20 segments with
