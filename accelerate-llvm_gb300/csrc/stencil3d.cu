@@ -102,7 +102,8 @@ stencil3d_kernel(const __grid_constant__ Stencil3Args a, const __grid_constant__
 //
 // A buffer row holds columns x0-PX .. x0+TW+PX-1 (PX = 16 bytes of elements,
 // so each row starts on a 16-byte boundary), copied in 16-byte pieces when the
-// array's rows are 16-byte aligned, else element by element; outside of the
+// array's rows are 16-byte aligned, else element by element (two adjacent outputs
+// leave in one store where the output's rows allow it); outside of the
 // array only columns -1 and w are read, each from its remapped place, and
 // cells under the constant boundary are written once.
 // PAT selects the taps at compile time: 0 = all 27 weights non-zero, 1 = the
@@ -145,7 +146,7 @@ template <class T> constexpr int s3_ctas() { return sizeof(T) == 4 ? 6 : 4; }
 template <class T, int PAT>
 __global__ void __launch_bounds__(S3S_THREADS, s3_ctas<T>())
 stencil3d_stream_kernel(const __grid_constant__ Stencil3Args a, const __grid_constant__ Stencil3W<T> W,
-                        int64_t zchunk, uint32_t mask, int vec) {
+                        int64_t zchunk, uint32_t mask, int vec, int pair) {
   constexpr int R = 1, K = 3, CE = s3_cols<T>();
   constexpr int S3S_STAGES = s3_stages<T>();
   constexpr int PX = 16 / (int)sizeof(T);             // left/right pad: one 16-byte piece
@@ -274,7 +275,7 @@ stencil3d_stream_kernel(const __grid_constant__ Stencil3Args a, const __grid_con
   // rows of this thread inside the array; columns likewise
   const int nrow = gyt + S3S_ROWS <= a.h ? S3S_ROWS : (int)(a.h - gyt > 0 ? a.h - gyt : 0);
   const int ncol = gx + CE <= a.w ? CE : (int)(a.w - gx > 0 ? a.w - gx : 0);
-  const bool whole = (CE == 1 || vec) && ncol == CE && nrow == S3S_ROWS;  // every output, 8-byte stores
+  const bool whole = (CE == 1 || pair) && ncol == CE && nrow == S3S_ROWS;  // every output, CE in one store
   T wr[K * K * K];  // the weights, in registers (read once from the parameter)
 #pragma unroll
   for (int t = 0; t < K * K * K; ++t) wr[t] = W.w[t];
@@ -397,11 +398,15 @@ int stencil3d_typed(const Stencil3Args &a, const void *weights, cudaStream_t s) 
       }
       const int64_t zchunk = s3_zchunk(sx * sy, a.d, (int64_t)device_info().sms * per_sm);
       const int64_t nz = cdiv_h(a.d, zchunk);
+      // 16-byte copies where every input row starts on such a boundary; 8-byte
+      // stores of two outputs where every pair of an output row does (the two
+      // arrays' alignments are independent of one another).
       const int vec = (reinterpret_cast<uintptr_t>(a.in) % 16 == 0) && ((a.w * (int64_t)sizeof(T)) % 16 == 0);
+      const int pair = (reinterpret_cast<uintptr_t>(a.out) % 8 == 0) && ((a.w * (int64_t)sizeof(T)) % 8 == 0);
       dim3 grid((unsigned)sx, (unsigned)sy, (unsigned)nz), block(S3S_TX, S3S_TY);
-      if (pat == 0) stencil3d_stream_kernel<T, 0><<<grid, block, 0, s>>>(a, W, zchunk, mask, vec);
-      else if (pat == 1) stencil3d_stream_kernel<T, 1><<<grid, block, 0, s>>>(a, W, zchunk, mask, vec);
-      else stencil3d_stream_kernel<T, 2><<<grid, block, 0, s>>>(a, W, zchunk, mask, vec);
+      if (pat == 0) stencil3d_stream_kernel<T, 0><<<grid, block, 0, s>>>(a, W, zchunk, mask, vec, pair);
+      else if (pat == 1) stencil3d_stream_kernel<T, 1><<<grid, block, 0, s>>>(a, W, zchunk, mask, vec, pair);
+      else stencil3d_stream_kernel<T, 2><<<grid, block, 0, s>>>(a, W, zchunk, mask, vec, pair);
       return check_launch();
     }
   }
