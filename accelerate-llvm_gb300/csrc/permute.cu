@@ -387,6 +387,25 @@ template <int OP, class T> constexpr bool split64() {
 // bin: lanes of a warp with the same key are added up first where keys repeat.
 template <int OP, class T> constexpr bool perm_aggregates() { return OP == ACC_ADD && is_fp<T>(); }
 
+// A private bin holds the combination of some of the updates without the
+// target's own value, which for the floats' + and * may leave the type's range
+// where no order that starts from the target does: 3e38 and 2e38 added to a
+// target of -3e38, or 1e30 twice with a target of 0.  Such a bin is not folded in;
+// its updates are applied to the target one by one instead, from a second read
+// of the CTA's share of the source.  For + the bin itself tells: an infinity or
+// NaN stays one.  For * a product that is not a normal number (zeros and lost bits
+// of subnormals, too) turns the bin into a NaN, which stays.
+template <int OP, class T> constexpr bool perm_redoes() { return is_fp<T>() && (OP == ACC_ADD || OP == ACC_MUL); }
+template <class T> __device__ __forceinline__ uint32_t exponent_bits(T v) {  // 0: zero, subnormal; all ones: inf, NaN
+  if constexpr (sizeof(T) == 4) return (__float_as_uint(v) >> 23) & 0xffu;
+  else return (uint32_t)((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffu;
+}
+template <class T> constexpr uint32_t exponent_ones() { return sizeof(T) == 4 ? 0xffu : 0x7ffu; }
+template <int OP, class T> __device__ __forceinline__ bool perm_redo(T bin) {
+  if constexpr (perm_redoes<OP, T>()) return exponent_bits(bin) == exponent_ones<T>();
+  else return false;
+}
+
 template <int OP, class T>
 __device__ __forceinline__ void private_update(unsigned char *bins, uint32_t m, uint32_t j, T x) {
   if constexpr (split64<OP, T>()) {
@@ -398,6 +417,18 @@ __device__ __forceinline__ void private_update(unsigned char *bins, uint32_t m, 
     } else if constexpr (OP == ACC_AND) { atomicAnd(lo, xl); atomicAnd(hi, xh); }
     else if constexpr (OP == ACC_OR) { atomicOr(lo, xl); atomicOr(hi, xh); }
     else { atomicXor(lo, xl); atomicXor(hi, xh); }
+  } else if constexpr (OP == ACC_MUL && is_fp<T>()) {
+    using U = typename std::conditional<sizeof(T) == 4, unsigned, unsigned long long>::type;
+    U *q = reinterpret_cast<U *>(bins) + j;
+    U old = *q, assumed;
+    do {
+      assumed = old;
+      T nv = Prim<OP, T>::ap(x, from_bits<T>(assumed));
+      const uint32_t e = exponent_bits(nv);
+      if (e == 0u || e == exponent_ones<T>()) nv = Prim<ACC_MAX, T>::id();  // NaN
+      if ((U)to_bits(nv) == assumed) break;
+      old = atomicCAS(q, assumed, (U)to_bits(nv));
+    } while (old != assumed);
   } else {
     atomic_combine<OP, T>(reinterpret_cast<T *>(bins) + j, x);
   }
@@ -410,6 +441,23 @@ __device__ __forceinline__ T private_bin(const unsigned char *bins, uint32_t m, 
   } else {
     return reinterpret_cast<const T *>(bins)[j];
   }
+}
+
+// The updates of the bins that were not folded in, one by one (a call of its
+// own: inlined, it cost the kernel around it registers).
+template <int OP, class T> __device__ __noinline__ void permute_redo(PermArgs a, const T *bins) {
+  const uint32_t m = (uint32_t)a.m;
+  T *out = static_cast<T *>(a.out);
+  using Unit = PermUnit<T>;
+  perm_stream<Unit, PERM_U>(a, from_bits<T>(a.cval), [&](const Unit (&q)[PERM_U]) {
+#pragma unroll
+    for (int u = 0; u < PERM_U; ++u)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int32_t j = q[u].j[k];
+        if ((uint32_t)j < m && perm_redo<OP, T>(bins[j])) atomic_combine<OP, T>(out + j, q[u].x[k]);
+      }
+  });
 }
 
 template <int OP, class T>
@@ -473,6 +521,7 @@ __global__ void __launch_bounds__(PERM_THREADS, 1) permute_private(PermArgs a) {
 
   // Fold this CTA's bins into the target; untouched bins hold the identity.
   T *out = static_cast<T *>(a.out);
+  bool redo = false;
   uint32_t b0 = 0;
   if constexpr (OP == ACC_ADD && std::is_same<T, float>::value) {
     // Four bins per reduction; an untouched bin takes -0.0, which changes nothing
@@ -495,7 +544,8 @@ __global__ void __launch_bounds__(PERM_THREADS, 1) permute_private(PermArgs a) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           const uint32_t mag = old[k] & 0x7fffffffu;
-          if (__float_as_uint(f[k]) != none) any = true;
+          if (perm_redo<OP, T>(f[k])) redo = apart = any = true;
+          else if (__float_as_uint(f[k]) != none) any = true;
           else if (mag - 1u < 0x007fffffu || mag > 0x7f800000u) apart = true;
         }
         if (!any) continue;
@@ -505,14 +555,18 @@ __global__ void __launch_bounds__(PERM_THREADS, 1) permute_private(PermArgs a) {
         } else {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
-            if (__float_as_uint(f[k]) != none) atomic_combine<OP, T>(out + b + k, f[k]);
+            if (__float_as_uint(f[k]) != none && !perm_redo<OP, T>(f[k])) atomic_combine<OP, T>(out + b + k, f[k]);
         }
       }
     }
   }
   for (uint32_t b = b0 + threadIdx.x; b < m; b += PERM_THREADS) {
     const T v = private_bin<OP, T>(smem_raw, m, b);
-    if (to_bits(v) != to_bits(idT)) atomic_combine<OP, T>(out + b, v);
+    if (perm_redo<OP, T>(v)) redo = true;
+    else if (to_bits(v) != to_bits(idT)) atomic_combine<OP, T>(out + b, v);
+  }
+  if constexpr (perm_redoes<OP, T>()) {
+    if (__syncthreads_or(redo)) permute_redo<OP, T>(a, reinterpret_cast<const T *>(smem_raw));
   }
 }
 
