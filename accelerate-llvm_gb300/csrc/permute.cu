@@ -273,6 +273,42 @@ __global__ void __launch_bounds__(256) permute_global(PermArgs a) {
 constexpr int PERM_THREADS = 1024;
 constexpr int PERM_U = 2;  // units of four elements per thread and round
 
+// A private bin holds the combination of some of the updates without the
+// target's own value, which for the floats' + and * may leave the type's range
+// where no order that starts from the target does: 3e38 and 2e38 added to a
+// target of -3e38, or 1e30 twice with a target of 0.  Such a bin is not folded in;
+// its updates are applied to the target one by one instead, from a second read
+// of the CTA's share of the source.  For + the bin itself tells: an infinity or
+// NaN stays one.  For * a product that is not a normal number (zeros and lost bits
+// of subnormals, too) turns the bin into a NaN, which stays.
+template <int OP, class T> constexpr bool perm_redoes() { return is_fp<T>() && (OP == ACC_ADD || OP == ACC_MUL); }
+template <class T> __device__ __forceinline__ uint32_t exponent_bits(T v) {  // 0: zero, subnormal; all ones: inf, NaN
+  if constexpr (sizeof(T) == 4) return (__float_as_uint(v) >> 23) & 0xffu;
+  else return (uint32_t)((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffu;
+}
+template <class T> constexpr uint32_t exponent_ones() { return sizeof(T) == 4 ? 0xffu : 0x7ffu; }
+template <int OP, class T> __device__ __forceinline__ bool perm_redo(T bin) {
+  if constexpr (perm_redoes<OP, T>()) return exponent_bits(bin) == exponent_ones<T>();
+  else return false;
+}
+
+// The updates of the bins that were not folded in, one by one (a call of its
+// own: inlined, it cost the kernel around it registers).
+template <int OP, class T> __device__ __noinline__ void permute_redo(PermArgs a, const T *bins) {
+  const uint32_t m = (uint32_t)a.m;
+  T *out = static_cast<T *>(a.out);
+  using Unit = PermUnit<T>;
+  perm_stream<Unit, PERM_U>(a, from_bits<T>(a.cval), [&](const Unit (&q)[PERM_U]) {
+#pragma unroll
+    for (int u = 0; u < PERM_U; ++u)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int32_t j = q[u].j[k];
+        if ((uint32_t)j < m && perm_redo<OP, T>(bins[j])) atomic_combine<OP, T>(out + j, q[u].x[k]);
+      }
+  });
+}
+
 // 32 bits per bin.  A counter may wrap mod 2^32 only beyond 2^32 updates per
 // CTA, where the 32-bit targets wrap as well and a 64-bit target's source
 // could not be in memory.
@@ -387,25 +423,6 @@ template <int OP, class T> constexpr bool split64() {
 // bin: lanes of a warp with the same key are added up first where keys repeat.
 template <int OP, class T> constexpr bool perm_aggregates() { return OP == ACC_ADD && is_fp<T>(); }
 
-// A private bin holds the combination of some of the updates without the
-// target's own value, which for the floats' + and * may leave the type's range
-// where no order that starts from the target does: 3e38 and 2e38 added to a
-// target of -3e38, or 1e30 twice with a target of 0.  Such a bin is not folded in;
-// its updates are applied to the target one by one instead, from a second read
-// of the CTA's share of the source.  For + the bin itself tells: an infinity or
-// NaN stays one.  For * a product that is not a normal number (zeros and lost bits
-// of subnormals, too) turns the bin into a NaN, which stays.
-template <int OP, class T> constexpr bool perm_redoes() { return is_fp<T>() && (OP == ACC_ADD || OP == ACC_MUL); }
-template <class T> __device__ __forceinline__ uint32_t exponent_bits(T v) {  // 0: zero, subnormal; all ones: inf, NaN
-  if constexpr (sizeof(T) == 4) return (__float_as_uint(v) >> 23) & 0xffu;
-  else return (uint32_t)((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffu;
-}
-template <class T> constexpr uint32_t exponent_ones() { return sizeof(T) == 4 ? 0xffu : 0x7ffu; }
-template <int OP, class T> __device__ __forceinline__ bool perm_redo(T bin) {
-  if constexpr (perm_redoes<OP, T>()) return exponent_bits(bin) == exponent_ones<T>();
-  else return false;
-}
-
 template <int OP, class T>
 __device__ __forceinline__ void private_update(unsigned char *bins, uint32_t m, uint32_t j, T x) {
   if constexpr (split64<OP, T>()) {
@@ -443,23 +460,6 @@ __device__ __forceinline__ T private_bin(const unsigned char *bins, uint32_t m, 
   }
 }
 
-// The updates of the bins that were not folded in, one by one (a call of its
-// own: inlined, it cost the kernel around it registers).
-template <int OP, class T> __device__ __noinline__ void permute_redo(PermArgs a, const T *bins) {
-  const uint32_t m = (uint32_t)a.m;
-  T *out = static_cast<T *>(a.out);
-  using Unit = PermUnit<T>;
-  perm_stream<Unit, PERM_U>(a, from_bits<T>(a.cval), [&](const Unit (&q)[PERM_U]) {
-#pragma unroll
-    for (int u = 0; u < PERM_U; ++u)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int32_t j = q[u].j[k];
-        if ((uint32_t)j < m && perm_redo<OP, T>(bins[j])) atomic_combine<OP, T>(out + j, q[u].x[k]);
-      }
-  });
-}
-
 template <int OP, class T>
 __global__ void __launch_bounds__(PERM_THREADS, 1) permute_private(PermArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -484,8 +484,8 @@ __global__ void __launch_bounds__(PERM_THREADS, 1) permute_private(PermArgs a) {
       // Every 8th round the warp looks at two of its updates: a key that three
       // lanes share turns the aggregation on (uniform keys over 256 bins do
       // that in 15 % of the looks, Zipf(1.1) keys in 85 %).  2 * 10^7 Float32
-      // values, uniform / Zipf keys over 5 * 10^4 bins: always 0.172 / 0.165
-      // ms, never 0.045 / 0.350 ms.
+      // values over 5 * 10^4 bins, when a lane still added its peers one by one:
+      // uniform keys always 0.172 ms, never 0.045; Zipf keys never 0.350.
       if ((round++ & 7u) == 0u) {
         const unsigned g0 = __match_any_sync(0xffffffffu, q[0].j[0]), g1 = __match_any_sync(0xffffffffu, q[PERM_U - 1].j[3]);
         const bool three = (q[0].j[0] >= 0 && __popc(g0) > 2) || (q[PERM_U - 1].j[3] >= 0 && __popc(g1) > 2);
@@ -502,13 +502,18 @@ __global__ void __launch_bounds__(PERM_THREADS, 1) permute_private(PermArgs a) {
         bool mine = (uint32_t)j < m;
         if constexpr (perm_aggregates<OP, T>()) {
           if (repeats) {  // warp-uniform
+            // pairwise in the order of the lanes: a key that every lane has
+            // takes 5 steps, not 31 (a lane that its partner has taken leaves the
+            // group).  2^22 sorted keys over 20,000 bins: Float32 66 -> 25 us,
+            // Float64 283 -> 72 (in L2 86); one key, Float32 73 -> 27.
             const unsigned grp = __match_any_sync(0xffffffffu, j);
-            unsigned rest = grp & (grp - 1u);  // the peers after the first lane
-            const T own = x;
+            const unsigned below = (1u << lane) - 1u;
+            unsigned rest = grp & ~below & ~(1u << lane), rank = __popc(grp & below);
             while (__any_sync(0xffffffffu, rest != 0u)) {
-              const T o = shfl_idx(own, rest ? __ffs(rest) - 1 : lane);
+              const T o = shfl_idx(x, rest ? __ffs(rest) - 1 : lane);
               if (rest) x = Prim<OP, T>::ap(x, o);
-              rest &= rest - 1u;
+              rest &= __ballot_sync(0xffffffffu, (rank & 1u) == 0u);
+              rank >>= 1;
             }
             mine = mine && (__ffs(grp) - 1) == lane;
           }
@@ -765,6 +770,30 @@ static int launch_count(const PermArgs &a, bool wide, size_t smem, int64_t per_c
               : launch_private(permute_count16<T, I64>, done16, smem, per_cta, a, s);
 }
 
+// Whether n updates of m bins go to private bins (which a CTA fills and folds
+// however few of its updates meet there) rather than to L2 one by one (where those
+// of one bin take 1.5 ns each).  Neither way is the better one for all keys, and the
+// keys are not known here; us of device time, private bins / L2:
+//   * 32-bit integers but *, one copy with native atomics: always.
+//   * 64-bit integers and every *: from 2^15 updates.  2^14 Int64 values into 2^10
+//     bins, uniform keys 7.1 / 4.2, Zipf keys 7.4 / 6.8; 2^15 into 2^9 uniform 6.8 /
+//     5.4, Zipf 7.3 / 11; 2^17 into 2^12 uniform 7.6 / 5.0, Zipf 7.8 / 29.
+//   * Float32 +: from 2^18, with 128 updates per bin from 2^16.  2^17 values into
+//     2^12 bins, uniform 9.9 / 6.8, Zipf 18.7 / 29.7; 2^18 into 2^13 10.4 / 6.4 and
+//     19.4 / 53; 2^16 into 2^8 13.6 / 17.3 and 17.7 / 21.5.
+//   * Float64 +: from 2^20.  2^18 into 2^12, uniform 14.7 / 6.5, Zipf 79 / 66; 2^20
+//     into 2^14 18.6 / 13.6 and 84 / 223.
+//   * min and max of floats, compare-and-swap loops either way: from 64 (Float64 128)
+//     updates per bin.  2^18 Float32 values into 2^13 bins, uniform 21 / 9.1, Zipf
+//     22 / 62; into 2^12 18.7 / 11.6 and 18.5 / 67.
+template <int OP, class T> static bool perm_private_pays(int64_t n, int64_t m) {
+  if constexpr (is_fp<T>() && (OP == ACC_MIN || OP == ACC_MAX)) return n >= (sizeof(T) == 4 ? 64 : 128) * m;
+  else if constexpr (is_fp<T>() && OP == ACC_ADD && sizeof(T) == 4) return n >= (1 << 18) || (n >= (1 << 16) && n >= 128 * m);
+  else if constexpr (is_fp<T>() && OP == ACC_ADD) return n >= (1 << 20);
+  else if constexpr (sizeof(T) == 8 || OP == ACC_MUL) return n >= (1 << 15);
+  else return true;
+}
+
 template <int OP, class T>
 int permute_typed(Workspace *w, PermArgs a, cudaStream_t s) {
   const Device &d = device_info();
@@ -780,7 +809,7 @@ int permute_typed(Workspace *w, PermArgs a, cudaStream_t s) {
   const int64_t smem_cap = d.max_smem_optin - 1024;
   const int64_t bytes = a.m * (int64_t)sizeof(T);
   const int64_t per_cta = 1024 * 8;
-  if (many && !force_global && !force_cluster) {
+  if (many && !force_global && !force_cluster && perm_private_pays<OP, T>(a.n, a.m)) {
     if constexpr (OP == ACC_ADD && !is_fp<T>()) {
       const bool wide = a.m * 4 <= smem_cap;
       if (!a.has_src && (a.m + 1) / 2 * 4 <= smem_cap) {
@@ -803,6 +832,10 @@ int permute_typed(Workspace *w, PermArgs a, cudaStream_t s) {
       if (a.m <= 8 * cap) return launch_permute_cluster<OP, T, 3>(a, agg, s);
     }
   }
+  // Four updates per thread from where one each nearly fills the machine; below, more
+  // threads are worth more than wider loads (2^17 Float32 max into 2^15 bins: 15.2 us by
+  // four, 7.0 by one; 2^19 into 2^15 15.7 and 21; 2^13 Int64 sums 4.2 and 3.5).
+  if (a.n < (1 << 19)) a.vec = 0;
   int64_t blocks = cdiv_h(a.vec ? cdiv_h(a.n, 4) : a.n, 256);
   if (blocks > (int64_t)d.sms * 16) blocks = (int64_t)d.sms * 16;
   permute_global<OP, T><<<(unsigned)blocks, 256, 0, s>>>(a);
