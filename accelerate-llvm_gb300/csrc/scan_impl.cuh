@@ -996,6 +996,9 @@ struct RowScanArgs {
 // with three barriers each:
 // 1001 x 4099 Float32, compensated, 16.6 -> 9.6 us; 600 x 8000 16.2 -> 10.4; 64
 // x 64,000 59 -> 17; 3000 x 100 Float64 42 -> 7.8.
+// Over a fused zipWith 12,000 x 4097 Float32 225 -> 109 us, 2000 x 4097 Int64 49 -> 35, over
+// a map 12,000 x 4097 Int32 103 -> 72 (327, 83 and 299 while each element was zipped as
+// it was loaded).
 constexpr int ROWS_MAXT = 1024;
 template <class T> constexpr int rows_k() { return sizeof(T) == 4 ? 16 : 8; }
 // 1-D arrays of at most one chunk take this kernel too, with one CTA: no tensor
@@ -1021,39 +1024,68 @@ __global__ void __launch_bounds__(ROWS_MAXT, 1) scan_rows_kernel(RowScanArgs a) 
   (void)mapc;
   const int64_t ch = (int64_t)nt * K;
   const int64_t nch = (a.inner + ch - 1) / ch;
-  // elements 0 * 32 + lane, 1 * 32 + lane, ... of this warp's part of chunk c of row r
-  auto load = [&](int64_t r, int64_t c, T (&x)[K]) {
+  // elements 0 * 32 + lane, 1 * 32 + lane, ... of this warp's part of chunk c of
+  // row r.  Zipped only when they are put into shared memory: zipped here, each
+  // element's load is waited for before the next one is issued.
+  auto load = [&](int64_t r, int64_t c, T (&x)[K], T (&y)[ZIP ? K : 1]) {
     const int64_t e0 = c * ch + warp * (32 * K) + lane;
     const T *src = static_cast<const T *>(a.in) + r * a.in_pitch + e0;
     const T *src2 = ZIP ? static_cast<const T *>(a.in2) + r * a.in_pitch + e0 : nullptr;
     (void)src2;
     const int64_t left = a.inner - e0;  // elements of the row from e0 on
-    auto elem = [&](int j) -> T {
-      if constexpr (ZIP) return zip_elem(a.zop, src[j * 32], src2[j * 32]);
-      else if constexpr (MAP) return zip_elem(a.zop, src[j * 32], mapc);
-      else return src[j * 32];
-    };
     if (left > 32 * (K - 1)) {
 #pragma unroll
-      for (int j = 0; j < K; ++j) x[j] = elem(j);
+      for (int j = 0; j < K; ++j) {
+        x[j] = src[j * 32];
+        if constexpr (ZIP) y[j] = src2[j * 32];
+      }
     } else {
 #pragma unroll
-      for (int j = 0; j < K; ++j) x[j] = j * 32 < left ? elem(j) : idT;
+      for (int j = 0; j < K; ++j) {
+        x[j] = j * 32 < left ? src[j * 32] : idT;
+        if constexpr (ZIP) y[j] = j * 32 < left ? src2[j * 32] : idT;
+      }
     }
   };
-  T next[K];
-  if ((int64_t)blockIdx.x < a.outer) load(blockIdx.x, R2L ? nch - 1 : 0, next);
+  // Chunk c's elements, into shared memory.
+  auto put = [&](int64_t c, const T (&x)[K], const T (&y)[ZIP ? K : 1]) {
+    if constexpr (ZIP || MAP) {
+      auto zipped = [&](auto zc) {
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+          turn[j * RPI * PITCH] = Prim<decltype(zc)::value, T>::ap(x[j], ZIP ? y[ZIP ? j : 0] : mapc);
+      };
+      switch (a.zop) {
+        case ACC_ADD: zipped(IC<ACC_ADD>{}); break;
+        case ACC_MUL: zipped(IC<ACC_MUL>{}); break;
+        case ACC_MIN: zipped(IC<ACC_MIN>{}); break;
+        default: zipped(IC<ACC_MAX>{}); break;
+      }
+      const int64_t left = a.inner - (c * ch + warp * (32 * K) + lane);
+      if (left <= 32 * (K - 1)) {
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+          if (j * 32 >= left) turn[j * RPI * PITCH] = idT;
+      }
+    } else {
+      (void)c;
+      (void)y;
+#pragma unroll
+      for (int j = 0; j < K; ++j) turn[j * RPI * PITCH] = x[j];
+    }
+  };
+  T next[K], next2[ZIP ? K : 1];
+  if ((int64_t)blockIdx.x < a.outer) load(blockIdx.x, R2L ? nch - 1 : 0, next, next2);
   int par = 0;
   for (int64_t r = blockIdx.x; r < a.outer; r += gridDim.x) {
     T *dst = static_cast<T *>(a.out) + r * a.out_pitch;
     S carry = a.has_seed ? A::lift(from_bits<T>(a.seed)) : A::id();
     for (int64_t ci = 0; ci < nch; ++ci, par ^= 1) {
       const int64_t c = R2L ? nch - 1 - ci : ci;
-#pragma unroll
-      for (int j = 0; j < K; ++j) turn[j * RPI * PITCH] = next[j];
+      put(c, next, next2);
       __syncwarp();
-      if (ci + 1 < nch) load(r, R2L ? c - 1 : c + 1, next);
-      else if (r + gridDim.x < a.outer) load(r + gridDim.x, R2L ? nch - 1 : 0, next);
+      if (ci + 1 < nch) load(r, R2L ? c - 1 : c + 1, next, next2);
+      else if (r + gridDim.x < a.outer) load(r + gridDim.x, R2L ? nch - 1 : 0, next, next2);
       S agg = A::lift(row[R2L ? K - 1 : 0]);
 #pragma unroll
       for (int j = 1; j < K; ++j) agg = A::push(agg, row[R2L ? K - 1 - j : j]);
