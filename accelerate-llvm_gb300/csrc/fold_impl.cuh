@@ -217,10 +217,11 @@ __global__ void __launch_bounds__(FOLD_LANE_WARPS * 32) fold_rows_lane(FoldArgs 
       }
     }
     __syncwarp();
-    typename A::S acc = A::lift(row[0]);
+    // from the seed on, as the rows of a thread are folded: values that leave the
+    // type's range without the seed need not with it
+    typename A::S acc = a.has_seed ? A::push(A::lift(from_bits<T>(a.seed)), row[0]) : A::lift(row[0]);
 #pragma unroll 4
     for (int j = 1; j < inner; ++j) acc = A::push(acc, row[j]);
-    if (a.has_seed) acc = A::comb(A::lift(from_bits<T>(a.seed)), acc);
     if (lane < rows) static_cast<T *>(a.out)[r0 + lane] = A::lower(acc);
     __syncwarp();
   }
