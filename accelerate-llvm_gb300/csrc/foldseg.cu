@@ -347,33 +347,50 @@ __global__ void foldseg_tile_index(const OT *off, int64_t nseg, int64_t ntiles, 
 // Complete the segment that closes at the first boundary of tile t0 + lane, for
 // 32 tiles (warp-collective): the carried-out values of the tiles since the
 // nearest earlier boundary, then the tile's own first part.  The previous tile
-// usually holds that boundary; where it does not, the warp walks back together,
-// 32 slots at a time.
-template <int OP, class T, int PREC>
+// usually holds that boundary.  Where it does not, a segmented scan over the warp
+// finds it within the 32, and one walk back over the slots before them serves all
+// that are open there: 32 slots at a time and, where all NT threads of a CTA call
+// (NT > 0), after 128 by the CTA together, 8 NT at a time.  One segment of 2^26 values
+// is 8192 tiles: 203 -> 110 us of device time (Float32, compensated), Int32 max 182 ->
+// 98; 5 * 10^6 Float32 values in 300 segments of two tiles 18.9 -> 13.0.
+template <int OP, class T, int PREC, int NT>
 __device__ __forceinline__ void seg_complete(const SegTileArgs &a, int64_t t0) {
   using A = Acc<OP, T, PREC>;
   using S = typename A::S;
   const int lane = threadIdx.x & 31;
   const int64_t t = t0 + lane;
   auto word = [&](const void *p) { return ld_relaxed_u64(static_cast<const uint64_t *>(p)); };
-  int64_t id = -1;
+  bool mine = false;
   S carry = A::id();
   bool closed = true;
   if (t < a.ntiles) {
     const SegSlot *prev = a.slots + (t > 0 ? t - 1 : 0);
-    id = (int64_t)word(&a.slots[t].first_id);
+    const int64_t id = (int64_t)word(&a.slots[t].first_id);
     const uint64_t pc = word(&prev->carry), pb = word(&prev->boundary);
-    if (id >= 0 && id < a.nseg && t > 0) {
+    mine = id >= 0 && id < a.nseg;
+    if (t > 0) {
       carry = from_bits<S>(pc);
       closed = pb != 0;
     }
   }
-  unsigned open = __ballot_sync(0xffffffffu, !closed);
-  while (open) {
-    const int l = __ffs(open) - 1;
-    open &= open - 1;
-    S acc = shfl_idx(carry, l);
-    for (int64_t k = t0 + l - 2;; k -= 32) {
+  const bool any_open = __any_sync(0xffffffffu, mine && !closed);
+  bool stopped = true;
+  if (any_open) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const S ov = shfl_up(carry, d);
+      const bool of = __shfl_up_sync(0xffffffffu, closed, d);
+      if (lane >= d && !closed) {
+        carry = A::comb(ov, carry);
+        closed = of;
+      }
+    }
+    stopped = !__any_sync(0xffffffffu, mine && !closed);
+  }
+  int64_t k = t0 - 2;  // the nearest slot that is not in `carry`
+  if (!stopped) {
+    S acc = A::id();
+    for (int i = 0; !stopped && (NT == 0 || i < 4); ++i, k -= 32) {
       const int64_t q = k - lane;
       S v = A::id();
       bool stop = q < 0;
@@ -382,22 +399,64 @@ __device__ __forceinline__ void seg_complete(const SegTileArgs &a, int64_t t0) {
         stop = word(&a.slots[q].boundary) != 0;
       }
       const unsigned sm = __ballot_sync(0xffffffffu, stop);
-      const int ks = sm ? __ffs(sm) - 1 : 32;
-      if (lane > ks) v = A::id();
-      const S w = shfl_idx(warp_reduce_rev<A>(v), 0);
-      acc = A::comb(w, acc);
-      if (sm) break;
+      if (lane > (sm ? __ffs(sm) - 1 : 32)) v = A::id();
+      acc = A::comb(shfl_idx(warp_reduce_rev<A>(v), 0), acc);
+      stopped = sm != 0u;
     }
-    if (lane == l) carry = acc;
+    if (!closed) carry = A::comb(acc, carry);
   }
-  if (t < a.ntiles && id >= 0 && id < a.nseg) {
+  if constexpr (NT > 0) {
+    if (__syncthreads_or(!stopped)) {
+      constexpr int U = 8, NW = NT / 32;
+      __shared__ S s_v[NW];
+      __shared__ int64_t s_from[NW];
+      __shared__ unsigned s_near[NW];
+      const int tid = threadIdx.x, warp = tid >> 5;
+      if (lane == 0) s_from[warp] = stopped ? -1 : k;
+      __syncthreads();
+      for (int w = 0; w < NW; ++w) {
+        S acc = A::id();
+        for (int64_t from = s_from[w]; from >= 0; from -= NT * U) {
+          S v[U];
+          unsigned near = NT * U;  // distance of the nearest slot that holds a boundary
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int64_t q = from - (u * NT + tid);
+            v[u] = A::id();
+            if (q < 0) continue;
+            v[u] = from_bits<S>(word(&a.slots[q].carry));
+            if (word(&a.slots[q].boundary) != 0 && near == NT * U) near = u * NT + tid;
+          }
+          near = __reduce_min_sync(0xffffffffu, near);
+          if (lane == 0) s_near[warp] = near;
+          __syncthreads();
+          for (int i = 0; i < NW; ++i) near = s_near[i] < near ? s_near[i] : near;
+          S sum = A::id();
+#pragma unroll
+          for (int u = U - 1; u >= 0; --u)
+            if ((unsigned)(u * NT + tid) <= near) sum = A::comb(sum, v[u]);
+          sum = warp_reduce_rev<A>(sum);
+          if (lane == 0) s_v[warp] = sum;
+          __syncthreads();
+          S all = s_v[NW - 1];
+          for (int i = NW - 2; i >= 0; --i) all = A::comb(all, s_v[i]);
+          acc = A::comb(all, acc);
+          __syncthreads();
+          if (near < NT * U) break;
+        }
+        if (w == warp && !closed) carry = A::comb(acc, carry);
+      }
+    }
+  }
+  if (mine) {
     const S v = A::comb(carry, from_bits<S>(word(&a.slots[t].first)));
-    static_cast<T *>(a.out)[id] = A::lower(a.has_seed ? A::comb(A::lift(from_bits<T>(a.seed)), v) : v);
+    static_cast<T *>(a.out)[word(&a.slots[t].first_id)] =
+        A::lower(a.has_seed ? A::comb(A::lift(from_bits<T>(a.seed)), v) : v);
   }
 }
 template <int OP, class T, int PREC>
 __global__ void __launch_bounds__(256) foldseg_fix(SegTileArgs a) {
-  seg_complete<OP, T, PREC>(a, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll);
+  seg_complete<OP, T, PREC, 256>(a, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll);
 }
 
 // ZIP: a thread zips its own rows of the two arrays' tiles in place before the walk.
@@ -597,7 +656,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a, cons
     if (s_bad != 2) return;
     __threadfence();
     if (tid == 0) *a.done = 0u;
-    for (int64_t t0 = warp * 32; t0 < a.ntiles; t0 += FT_THREADS) seg_complete<OP, T, PREC>(a, t0);
+    for (int64_t t0 = warp * 32; t0 < a.ntiles; t0 += FT_THREADS) seg_complete<OP, T, PREC, 0>(a, t0);
   };
   // A tile whose load never landed is not read.
   if (__syncthreads_or(!landed)) {
