@@ -459,12 +459,15 @@ __global__ void __launch_bounds__(256) foldseg_fix(SegTileArgs a) {
   seg_complete<OP, T, PREC, 256>(a, (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~31ll);
 }
 
-// ZIP: a thread zips its own rows of the two arrays' tiles in place before the walk.
+// ZIP: a thread zips its own rows of the two arrays' tiles in place before the
+// walk, its 16-byte pieces in an order of its own (both rows are swizzled alike): all
+// lanes on one column would meet on the same banks.
 template <class T, int Z>
-__device__ __forceinline__ void seg_zip_row(unsigned char *row, const unsigned char *row2) {
+__device__ __forceinline__ void seg_zip_row(unsigned char *row, const unsigned char *row2, int order) {
   constexpr int VEC = 16 / sizeof(T);
 #pragma unroll
-  for (int c = 0; c < FT_ROW_BYTES / 16; ++c) {  // in whatever order: both rows are swizzled alike
+  for (int i = 0; i < FT_ROW_BYTES / 16; ++i) {
+    const int c = i ^ order;
     uint4 v = reinterpret_cast<const uint4 *>(row)[c];
     const uint4 w = reinterpret_cast<const uint4 *>(row2)[c];
     T x[VEC], y[VEC];
@@ -667,10 +670,10 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a, cons
     unsigned char *row = buf + tid * FT_ROW_BYTES;
     const unsigned char *row2 = row + SUB_BYTES;
     switch (a.zop) {
-      case ACC_ADD: seg_zip_row<T, ACC_ADD>(row, row2); break;
-      case ACC_MUL: seg_zip_row<T, ACC_MUL>(row, row2); break;
-      case ACC_MIN: seg_zip_row<T, ACC_MIN>(row, row2); break;
-      default: seg_zip_row<T, ACC_MAX>(row, row2); break;
+      case ACC_ADD: seg_zip_row<T, ACC_ADD>(row, row2, tid & 7); break;
+      case ACC_MUL: seg_zip_row<T, ACC_MUL>(row, row2, tid & 7); break;
+      case ACC_MIN: seg_zip_row<T, ACC_MIN>(row, row2, tid & 7); break;
+      default: seg_zip_row<T, ACC_MAX>(row, row2, tid & 7); break;
     }
   }
   // The values after the last whole row (TMA left zeros there; the positions
