@@ -261,7 +261,8 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 // 19,800 (2^22 values); the tiles now wait for no one.  2^26 Float32 values in
 // 2^20 lognormal segments, compensated: 115 -> 92 us, plain 88 -> 76, Int32 max
 // 88 -> 76 (the index pre-pass is about 5 of them, the completion 3).
-constexpr int FT_THREADS = 128;
+// DENSE: the tiles of short segments (see ft_dense), 256 threads with one row.
+template <bool DENSE = false> constexpr int ft_threads() { return DENSE ? 256 : 128; }
 constexpr int FT_ROW_BYTES = 128;
 // Tile-relative offsets (and their results) held in shared memory: the walk by
 // boundary slots needs all of a tile's, so segments of 11 values and more on
@@ -275,7 +276,13 @@ constexpr int FT_CAP = 768;
 // (76), 2^26 Int32 values in segments of 16 231 (110: 16,384 values have more
 // boundaries than are kept), 2^25 Float64 140 (116).
 // Over a fused zipWith each tile needs the rows of both arrays: one row each.
-template <bool ZIP> constexpr int ft_rpt() { return ZIP ? 1 : 2; }
+template <bool ZIP, bool DENSE = false> constexpr int ft_rpt() { return ZIP || DENSE ? 1 : 2; }
+
+// Segments of fewer than 11 values on average leave a tile more offsets than are
+// kept, and its threads walk value by value; a thread then carries a compensated
+// state over one row only (2^24 Float32 values, compensated, against two: segments of
+// 2 197 -> 121 us, of 6 94 -> 66, of 10 73 -> 56, of 12 39 and 41; other states gain nothing).
+template <class S> constexpr bool ft_dense() { return std::is_same<S, F2>::value; }
 
 struct SegTileArgs {
   const void *in;
@@ -313,8 +320,11 @@ constexpr int TIDX_SHIFT = 35;  // offset indices below 2^35; the epoch above
 // -> 11.1.  At the limits, 10^6 Float32 values: 4,000 segments by offsets 14.8 ->
 // 13.2 us, 15,625 segments (three launches) 15.0 -> 12.1.
 constexpr int FT_SMALL = 4096;
-constexpr int FT_PER = (FT_SMALL + FT_THREADS) / FT_THREADS;  // most offsets per thread
-static_assert(FT_PER % 2 == 1 && FT_PER * FT_THREADS >= FT_SMALL + 1, "an odd number (free of bank conflicts) holds them all");
+// most offsets per thread
+template <bool DENSE> constexpr int ft_per() { return (FT_SMALL + ft_threads<DENSE>()) / ft_threads<DENSE>(); }
+static_assert(ft_per<false>() % 2 == 1 && ft_per<false>() * ft_threads<false>() >= FT_SMALL + 1 &&
+                  ft_per<true>() % 2 == 1 && ft_per<true>() * ft_threads<true>() >= FT_SMALL + 1,
+              "an odd number (free of bank conflicts) holds them all");
 
 // Pre-pass: tidx[t] = the first k with off[k] >= t << log_te (t < ntiles), and
 // tidx[ntiles] = nseg + 1, each tagged with the call's epoch so that no
@@ -480,12 +490,13 @@ __device__ __forceinline__ void seg_zip_row(unsigned char *row, const unsigned c
   }
 }
 
-template <int OP, class T, int PREC, class OT, bool ZIP = false>
-__global__ void __launch_bounds__(FT_THREADS, ZIP ? 4 : 5)
+template <int OP, class T, int PREC, class OT, bool ZIP = false, bool DENSE = false>
+__global__ void __launch_bounds__(ft_threads<DENSE>(), ZIP ? 4 : 5)
 foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a, const __grid_constant__ CUtensorMap tin2) {
   using A = Acc<OP, T, PREC>;
   using S = typename A::S;
-  constexpr int FT_RPT = ft_rpt<ZIP>();
+  constexpr int FT_THREADS = ft_threads<DENSE>(), FT_PER = ft_per<DENSE>();
+  constexpr int FT_RPT = ft_rpt<ZIP, DENSE>();
   constexpr int ITEMS = FT_ROW_BYTES / sizeof(T);
   constexpr int VEC = 16 / sizeof(T);
   constexpr int W = FT_RPT * ITEMS;          // values per thread (FT_RPT adjacent rows)
@@ -923,14 +934,14 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a, cons
 
 // One launcher per kernel instantiation, so that each gets its own
 // shared-memory attribute (the tile needs more than the default 48 KB).
-template <int OP, class T, int PREC, class OT, bool ZIP>
+template <int OP, class T, int PREC, class OT, bool ZIP, bool DENSE>
 int launch_foldseg_tile(const CUtensorMap &tin, const SegTileArgs &a, int64_t ntiles, cudaStream_t s,
                         const CUtensorMap &tin2) {
-  constexpr int FT_RPT = ft_rpt<ZIP>();
+  constexpr int FT_THREADS = ft_threads<DENSE>(), FT_PER = ft_per<DENSE>(), FT_RPT = ft_rpt<ZIP, DENSE>();
   const size_t tile = (size_t)(ZIP ? 2 : 1) * FT_RPT * FT_THREADS * FT_ROW_BYTES + 1024;
   const size_t all = (size_t)(FT_PER * FT_THREADS + FT_THREADS / 32) * sizeof(OT);  // small: the offsets, the warps' sums
   const size_t smem = tile + (a.small ? all : 0);
-  auto kern = foldseg_tile_kernel<OP, T, PREC, OT, ZIP>;
+  auto kern = foldseg_tile_kernel<OP, T, PREC, OT, ZIP, DENSE>;
   static std::atomic<uint64_t> attr_done{0};
   smem_attrs_once(kern, (int)(tile + all), attr_done);
   kern<<<(unsigned)ntiles, FT_THREADS, smem, s>>>(tin, a, tin2);
@@ -940,7 +951,7 @@ int launch_foldseg_tile(const CUtensorMap &tin, const SegTileArgs &a, int64_t nt
   return check_launch();
 }
 
-template <int OP, class T, int PREC, bool ZIP = false>
+template <int OP, class T, int PREC, bool ZIP = false, bool DENSE = false>
 int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bool lengths, T *out, int64_t inner,
                        int64_t nseg, bool has_seed, uint64_t seed, cudaStream_t s, bool *taken,
                        const T *in2 = nullptr, int zop = 0) {
@@ -951,8 +962,13 @@ int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bo
   // lanes wait for the longest, gain more than equal ones lose: 2^24 Float64 values in
   // segments of 20, lognormal 254 (118), equal 81 (114).
   if (ZIP && inner < 16 * nseg) return ACC_OK;
+  if constexpr (!DENSE && !ZIP && ft_dense<typename Acc<OP, T, PREC>::S>()) {
+    if (inner < 11 * nseg)
+      return foldseg_tile_typed<OP, T, PREC, ZIP, true>(w, in, off, off64, lengths, out, inner, nseg, has_seed, seed, s,
+                                                        taken);
+  }
   constexpr int ITEMS = FT_ROW_BYTES / sizeof(T);
-  constexpr int FT_RPT = ft_rpt<ZIP>();
+  constexpr int FT_THREADS = ft_threads<DENSE>(), FT_RPT = ft_rpt<ZIP, DENSE>();
   constexpr int64_t TE = (int64_t)FT_THREADS * FT_RPT * ITEMS;
   constexpr int LOG_TE = 31 - __builtin_clz((unsigned)TE);
   static_assert(TE == int64_t(1) << LOG_TE, "tiles of a power of two values");
@@ -1005,8 +1021,8 @@ int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bo
     st = check_launch();
     if (st) return st;
   }
-  return off64 ? launch_foldseg_tile<OP, T, PREC, int64_t, ZIP>(tin, a, ntiles, s, tin2)
-               : launch_foldseg_tile<OP, T, PREC, int32_t, ZIP>(tin, a, ntiles, s, tin2);
+  return off64 ? launch_foldseg_tile<OP, T, PREC, int64_t, ZIP, DENSE>(tin, a, ntiles, s, tin2)
+               : launch_foldseg_tile<OP, T, PREC, int32_t, ZIP, DENSE>(tin, a, ntiles, s, tin2);
 }
 
 // ----------------------------------------------------------------- host side
