@@ -511,35 +511,49 @@ static std::map<TuneKey, TuneVal> g_tune;
 
 static bool valid_nt(int nt) { return nt == 128 || nt == 256 || nt == 512; }
 static int type_bytes(int type) { return (type == ACC_I64 || type == ACC_F64) ? 8 : 4; }
-// Elements per thread as the kernel takes them: 16 or 64 bytes' worth, the
-// nearer one.
+// Elements per thread as the kernel takes them: 16 or 64 bytes' worth.  32 bytes, which
+// tables and other launch shapes ask for, round up (1000 requests of 2^8 .. 2^22
+// elements at 512 threads: 654 us with 16 bytes for those below a megabyte, 589 with 64).
 static int norm_ipt(int ipt, int type) {
   const int eb = type_bytes(type);
-  return B_BYTES[ipt * eb > 32 ? 1 : 0] / eb;
+  return B_BYTES[ipt * eb >= 32 ? 1 : 0] / eb;
 }
 static int bucket_of(int64_t n) {
   int b = 0;
   while (b < 62 && (int64_t(1) << (b + 1)) <= n) ++b;
   return b;
 }
-static int default_ipt(int kind, int type, int64_t n) {
-  (void)kind;
-  return B_BYTES[n * type_bytes(type) > BT * B_BYTES[0] ? 1 : 0] / type_bytes(type);
+// Before tuning: the narrow tile where it holds the whole request.
+static int default_ipt(int type, int64_t n, int nt) {
+  return B_BYTES[n * type_bytes(type) > nt * B_BYTES[0] ? 1 : 0] / type_bytes(type);
 }
-static TuneVal tuned(int kind, int type, int64_t n) {
+// Before tuning, a request's threads per CTA:
+//   * 128 up to 8 KB: more requests are in work at once (2000 scans of 2^8 Int32 / Float32
+//     elements 11.0 / 13.7 -> 8.2 / 9.5 us of device time, of 2^10 Int64 15.4 -> 10.9; the tiles
+//     of 2^12, 16 KB, are faster with 256: 17 and 19);
+//   * 512 from a megabyte on: larger tiles, so fewer look-backs (1000 requests of 2^8 ..
+//     2^22 elements 627 -> 589 us, one scan of 2^20 Float32 9.1 -> 8.0);
+//   * 256 otherwise, and for Float64, whose additions bind it (500 scans of 2^17 545 us
+//     with 512, 480 with 256).
+static int default_nt(int type, int64_t n) {
+  const int64_t bytes = n * type_bytes(type);
+  if (bytes <= 8192) return 128;
+  return type != ACC_F64 && bytes >= (1 << 20) ? 512 : BT;
+}
+// The request's entry of the tuning table, if it has one.
+static bool tuned(int kind, int type, int64_t n, TuneVal *v) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   auto it = g_tune.find(TuneKey{kind, type, bucket_of(n)});
-  if (it != g_tune.end()) return it->second;
-  // Before tuning, requests of a megabyte and more ask for 512 threads: larger
-  // tiles, so fewer look-backs (0.60 ms against 0.64 for 1000 requests whose
-  // bytes are mostly in such; 36 small ones take 0.017 ms either way).
-  return TuneVal{default_ipt(kind, type, n), n * type_bytes(type) >= (1 << 20) ? 512 : BT};
+  if (it == g_tune.end()) return false;
+  *v = it->second;
+  return true;
 }
 // A request's elements per thread in a launch of nt threads: its tuned tile
 // shape where the tuned launch shape is nt, else the same tile size in
 // elements.
 static int ipt_for(const acc_request &q, int nt) {
-  const TuneVal v = tuned(q.kind, q.type, q.n);
+  TuneVal v;
+  if (!tuned(q.kind, q.type, q.n, &v)) return default_ipt(q.type, q.n, nt);
   const int ipt = v.nt == nt ? v.ipt : (int)(((int64_t)v.ipt * v.nt) / nt);
   return norm_ipt(ipt, q.type);
 }
@@ -617,16 +631,26 @@ static int batch_make(int op, const acc_request *reqs, int64_t count, const int3
     if (!valid_nt(nt_override)) return ACC_ERR_INVALID;
     nt = nt_override;
   } else {
-    double weight[3] = {0.0, 0.0, 0.0};
+    double weight[3] = {0.0, 0.0, 0.0}, folds = 0.0;
+    int64_t wide_items = 0;  // folds' items at 512 threads
     for (int64_t i = 0; i < count; ++i) {
       const acc_request &q = reqs[i];
       if (q.type != ACC_I32 && q.type != ACC_I64 && q.type != ACC_F32 && q.type != ACC_F64) continue;
-      const int v = tuned(q.kind, q.type, q.n).nt;
+      const double bytes = (double)(q.n > 0 ? q.n : 0) * type_bytes(q.type);
+      TuneVal v{0, default_nt(q.type, q.n)};
+      const bool table = tuned(q.kind, q.type, q.n, &v);
       for (int c = 0; c < 3; ++c)
-        if (B_NT[c] == v) weight[c] += (double)(q.n > 0 ? q.n : 0) * type_bytes(q.type);
+        if (B_NT[c] == v.nt) weight[c] += bytes;
+      if (q.kind == ACC_REQ_FOLD && !table && q.n > 0) {
+        folds += bytes;
+        wide_items += cdiv_h(q.n, item_elems(q, default_ipt(q.type, q.n, 512), 512));
+      }
     }
     if (weight[0] > weight[1] && weight[0] >= weight[2]) nt = B_NT[0];
     else if (weight[2] > weight[1] && weight[2] > weight[0]) nt = B_NT[2];
+    // Untuned folds that leave SMs without one of 512 threads' items take 256 (one fold of
+    // 2^20 Float32 values 8.4 -> 7.2 us, of 2^18 Float64 12.1 -> 9.3).
+    if (nt == B_NT[2] && folds > 0.5 * (weight[0] + weight[1] + weight[2]) && wide_items < device_info().sms) nt = BT;
   }
   std::vector<BReq> h(count);
   std::vector<int32_t> item_req;
@@ -807,7 +831,7 @@ static int autotune_run(int kind, int type, int bucket, cudaStream_t s, void *bu
     q.out = base + (size_t)n * eb + (kind == ACC_REQ_SCAN ? (size_t)i * n * eb : (size_t)i * eb);
   }
   float best_ms = 1e30f;
-  TuneVal pick{default_ipt(kind, type, n), BT};
+  TuneVal pick{default_ipt(type, n, BT), BT};
   // every launch shape, and for each every tile shape
   for (int nt : B_NT) {
     for (int bytes : B_BYTES) {
