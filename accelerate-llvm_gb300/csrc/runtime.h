@@ -138,6 +138,20 @@ inline void smem_attrs_once(K kern, int bytes, std::atomic<uint64_t> &done, bool
   done.fetch_or(bit, std::memory_order_release);
 }
 
+// A kernel's resident CTAs per SM, asked for (`ask`) once per device: devices may
+// differ, and a cooperative grid sized for another one does not launch.  Not kept
+// where the question fails (0).
+using ResidentCache = std::atomic<int>[64];
+template <class F> int resident_once(ResidentCache &cache, F &&ask) {
+  const int dev = device_info().id;
+  const bool keep = dev >= 0 && dev < 64;
+  int n = keep ? cache[dev].load(std::memory_order_relaxed) : 0;
+  if (n > 0) return n;
+  n = ask();
+  if (n > 0 && keep) cache[dev].store(n, std::memory_order_relaxed);
+  return n > 0 ? n : 0;
+}
+
 // Fill n elements with one value (the seed fill of empty folds and scans,
 // the reference's `generate` of the seed, PTX/CodeGen/Generate.hs:40-61).
 template <class T> int launch_fill(T *out, int64_t n, uint64_t bits, cudaStream_t s);

@@ -1211,15 +1211,14 @@ int launch_scan_l2(Workspace *w, const T *in, T *out, T *total_out, T *seed_out,
   auto kern = scan_l2_kernel<OP, T, PREC, R2L, PROD, SEG>;
   static std::atomic<uint64_t> attr_done{0};
   smem_attrs_once(kern, (int)smem, attr_done);
-  static std::atomic<int> resident{0};  // CTAs per SM, asked for once
-  int per_sm = resident.load(std::memory_order_relaxed);
-  if (per_sm == 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, L2S_THREADS, smem) != cudaSuccess || per_sm < 1) {
-      cudaGetLastError();
-      return ACC_OK;
-    }
-    resident.store(per_sm, std::memory_order_relaxed);
-  }
+  static ResidentCache resident{};
+  const int per_sm = resident_once(resident, [&] {
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, L2S_THREADS, smem) == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
+  });
+  if (per_sm == 0) return ACC_OK;
   int st = ws_status(w, (size_t)ntiles * 2);
   if (st) return st;
   ScanArgs a{};

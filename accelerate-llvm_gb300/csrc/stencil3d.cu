@@ -389,13 +389,14 @@ int stencil3d_typed(const Stencil3Args &a, const void *weights, cudaStream_t s) 
       const void *fn = pat == 0 ? (const void *)stencil3d_stream_kernel<T, 0>
                        : pat == 1 ? (const void *)stencil3d_stream_kernel<T, 1>
                                   : (const void *)stencil3d_stream_kernel<T, 2>;
-      static std::atomic<int> resident_ctas[3];
-      int per_sm = resident_ctas[pat].load(std::memory_order_relaxed);
-      if (per_sm == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, S3S_THREADS, 0) != cudaSuccess || per_sm < 1)
-          per_sm = 1;
-        resident_ctas[pat].store(per_sm, std::memory_order_relaxed);
-      }
+      static ResidentCache resident[3]{};
+      int per_sm = resident_once(resident[pat], [&] {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, S3S_THREADS, 0) == cudaSuccess) return n;
+        cudaGetLastError();
+        return 0;
+      });
+      if (per_sm == 0) per_sm = 1;
       const int64_t zchunk = s3_zchunk(sx * sy, a.d, (int64_t)device_info().sms * per_sm);
       const int64_t nz = cdiv_h(a.d, zchunk);
       // 16-byte copies where every input row starts on such a boundary; 8-byte
