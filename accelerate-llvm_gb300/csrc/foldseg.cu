@@ -254,7 +254,8 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 // An extra tile past the last value closes the segments that end at the very
 // end of the row.  Three launches: the index pre-pass, the tiles and the
 // completion; one for short calls.  Offsets that decrease or leave [0, n] raise
-// ACC_ERR_INDEX; the tile then writes nothing.
+// ACC_ERR_INDEX; of a tile that holds such offsets only the z of empty segments may
+// have been written, inside of the output.
 // Bound: issue (about 30 thread instructions per value, compensated).  A tile
 // that completed its first segment itself, by a decoupled look-back, held its
 // shared memory for 7,400 cycles of polls and 2,100 of drawing a ticket, of

@@ -612,16 +612,17 @@ template <int OP, class T> __device__ __forceinline__ T agg_value(T x, int cnt) 
 template <int OP, class T, int LOG_CL, bool AGG>
 __global__ void __launch_bounds__(1024, 1) permute_cluster(PermArgs a, int per) {
   constexpr int CL = 1 << LOG_CL;
+  static_assert(CL > 1 && CL <= 8, "a portable cluster");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T *bins = reinterpret_cast<T *>(smem_raw);
-  const uint32_t rank = CL > 1 ? cg::this_cluster().block_rank() : 0u;
+  const uint32_t rank = cg::this_cluster().block_rank();
   const T idT = Prim<OP, T>::id();
   for (int b = threadIdx.x; b < per; b += blockDim.x) bins[b] = idT;
-  if constexpr (CL > 1) cg::this_cluster().sync(); else __syncthreads();
+  cg::this_cluster().sync();
   const uint32_t bins_addr = smem_addr(bins);
   uint32_t remote_base[CL];
 #pragma unroll
-  for (int r = 0; r < CL; ++r) remote_base[r] = CL > 1 ? mapa_shared(bins_addr, (uint32_t)r) : bins_addr;
+  for (int r = 0; r < CL; ++r) remote_base[r] = mapa_shared(bins_addr, (uint32_t)r);
 
   const T *src = static_cast<const T *>(a.src);
   const T c = from_bits<T>(a.cval);
@@ -685,7 +686,7 @@ __global__ void __launch_bounds__(1024, 1) permute_cluster(PermArgs a, int per) 
     }
   }
   if (bad) raise_error(a.err, DEV_ERR_INDEX);
-  if constexpr (CL > 1) cg::this_cluster().sync(); else __syncthreads();
+  cg::this_cluster().sync();
 
   // Fold this CTA's bins into the target; untouched bins hold the identity.
   T *out = static_cast<T *>(a.out);
@@ -698,7 +699,8 @@ __global__ void __launch_bounds__(1024, 1) permute_cluster(PermArgs a, int per) 
 
 // ----------------------------------------------------------------- host side
 // Variant choice (tuning knob, default "auto"): ACC_GB300_PERMUTE = auto |
-// cluster | global, ACC_GB300_PERMUTE_AGG = 0 | 1 (the cluster kernel's).
+// cluster | global (anything else is auto), ACC_GB300_PERMUTE_AGG = 0 | 1 (the
+// cluster kernel's).
 static int env_int(const char *name, int dflt) {
   const char *v = getenv(name);
   return v ? atoi(v) : dflt;
@@ -713,7 +715,6 @@ static int launch_cluster(K kern, int CL, unsigned threads, size_t smem, int64_t
                           Args... args) {
   const Device &d = device_info();
   cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (CL > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

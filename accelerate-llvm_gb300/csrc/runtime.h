@@ -26,7 +26,8 @@ struct Workspace {
   int device = -1;
   cudaStream_t stream = nullptr;
   // Small always-zero-between-calls area: [0] error word, [1] scan tile
-  // ticket, [2] foldSeg big-segment count, [3..] per-row fold tickets.
+  // ticket, [2] foldSeg big-segment count, [3] blocks that have finished, [8..]
+  // per-row fold tickets.
   uint32_t *words = nullptr;
   size_t nwords = 0;
   // Look-back status slots (2 x u64 per tile), tagged with an epoch.

@@ -1449,8 +1449,6 @@ template <int OP, class T, int PREC, bool R2L, bool MAP = false>
 int launch_scan_1d(Workspace *w, const T *in, T *out, T *total_out, T *seed_out, int64_t n,
                    bool has_seed, bool exclusive, uint64_t seed, cudaStream_t s, int mop = 0,
                    uint64_t mapc = 0) {
-  // Arrays of at least four 32 KiB tiles per SM take the persistent
-  // L2-re-read kernel (ACC_GB300_SCAN_KERNEL=tile keeps the tile kernel).
   if (n <= rows_1d<T>()) {
     RowScanArgs a{};
     a.in = in; a.out = out; a.sums = total_out;
@@ -1460,6 +1458,8 @@ int launch_scan_1d(Workspace *w, const T *in, T *out, T *total_out, T *seed_out,
     a.zop = mop; a.mapc = mapc;
     return launch_scan_rows<OP, T, PREC, R2L, false, MAP>(a, s);
   }
+  // Arrays of at least four 32 KiB tiles per SM take the persistent
+  // L2-re-read kernel (ACC_GB300_SCAN_KERNEL=tile keeps the tile kernel).
   static const bool l2k = !(getenv("ACC_GB300_SCAN_KERNEL") && strcmp(getenv("ACC_GB300_SCAN_KERNEL"), "tile") == 0);
   if (l2k && n * (int64_t)sizeof(T) >= (int64_t)device_info().sms * 4 * L2S_TILE) {
     bool launched = false;

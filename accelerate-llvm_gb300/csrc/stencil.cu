@@ -143,17 +143,16 @@ stencil_kernel(const __grid_constant__ CUtensorMap tin, StencilArgs a, StencilW<
   }
 }
 
-// ----------------------------------------------------------------- specialised sweep
-// The same computation with the radii and the tap pattern known at compile
-// time: PAT 0 = every tap has a non-zero weight, PAT 1 = the cross (5-point
+// ----------------------------------------------------------------- second pass
+// The second pass of stencil2 for the usual radii: the same computation from the
+// accumulators in `out`, with the radii and the tap pattern known at compile time: PAT 0 = every tap has a non-zero weight, PAT 1 = the cross (5-point
 // style: only the corners of the 3x3 are zero), PAT 2 = any pattern (each tap
 // tested against a zero mask).  Tiles are 64 x 64 outputs, 16 rows per thread.
 constexpr int SF_TW = 64, SF_TH = 64, SF_ROWS = 16;
 
 template <class T, int RY, int RX, int PAT>
 __global__ void __launch_bounds__(ST_THREADS, (sizeof(T) == 4 && RY * RX <= 1) ? 4 : 2)
-stencil_fast_kernel(const __grid_constant__ CUtensorMap tin, StencilArgs a, StencilW<T> W, uint32_t zmask_lo,
-                    uint32_t zmask_hi) {
+stencil_onto_kernel(const __grid_constant__ CUtensorMap tin, StencilArgs a, StencilW<T> W, uint32_t zmask) {
   constexpr int PX = ((RX * (int)sizeof(T) + 15) / 16) * 16 / (int)sizeof(T) > 0
                          ? ((RX * (int)sizeof(T) + 15) / 16) * 16 / (int)sizeof(T) : 0;
   constexpr int SW = SF_TW + 2 * PX;
@@ -213,7 +212,7 @@ stencil_fast_kernel(const __grid_constant__ CUtensorMap tin, StencilArgs a, Sten
 #pragma unroll
   for (int r = 0; r < SF_ROWS; ++r) {
     const int64_t gy = ty0 + oy0 + r;
-    acc[r] = (a.accumulate && gy < a.h && gx < a.w) ? out[gy * a.out_pitch + gx] : Prim<ACC_ADD, T>::id();
+    acc[r] = gy < a.h && gx < a.w ? out[gy * a.out_pitch + gx] : Prim<ACC_ADD, T>::id();
   }
   const T *trow = tile + oy0 * SW + PX + col;  // smem row oy0 - RY + RY = oy0 (halo offset)
 #pragma unroll
@@ -232,8 +231,7 @@ stencil_fast_kernel(const __grid_constant__ CUtensorMap tin, StencilArgs a, Sten
           if (k == 0 || k == 2 || k == 6 || k == 8) continue;  // corners of the 3x3 cross
         }
         if constexpr (PAT == 2) {
-          const bool zero = k < 32 ? ((zmask_lo >> k) & 1u) : ((zmask_hi >> (k - 32)) & 1u);
-          if (zero) continue;
+          if ((zmask >> k) & 1u) continue;
         }
         acc[r] = fma_tap(w[k], xv[dx], acc[r]);
       }
@@ -247,7 +245,7 @@ stencil_fast_kernel(const __grid_constant__ CUtensorMap tin, StencilArgs a, Sten
 }
 
 template <class T, int RY, int RX, int PAT>
-int stencil_fast_launch(StencilArgs a, const StencilW<T> &W, uint32_t zlo, uint32_t zhi, cudaStream_t s) {
+int stencil_onto_launch(StencilArgs a, const StencilW<T> &W, uint32_t zmask, cudaStream_t s) {
   constexpr int PX = ((RX * (int)sizeof(T) + 15) / 16) * 16 / (int)sizeof(T);
   constexpr int SW = SF_TW + 2 * PX;
   constexpr int SH = SF_TH + 2 * RY;
@@ -256,12 +254,12 @@ int stencil_fast_launch(StencilArgs a, const StencilW<T> &W, uint32_t zlo, uint3
   memset(&tin, 0, sizeof(tin));
   a.tma = encode_2d(&tin, a.in, sizeof(T), (uint64_t)a.in_w, (uint64_t)a.in_h, (uint64_t)a.in_pitch * sizeof(T),
                     SW, SH, false);
-  auto kern = stencil_fast_kernel<T, RY, RX, PAT>;
+  auto kern = stencil_onto_kernel<T, RY, RX, PAT>;
   static std::atomic<uint64_t> attr_done{0};
   smem_attrs_once(kern, (int)smem, attr_done, false);
   const int64_t gx = cdiv_h(a.w, SF_TW), gy = cdiv_h(a.h, SF_TH);
   if (gy > 65535 || gx > (1ll << 31) - 1) return ACC_ERR_TOO_LARGE;
-  kern<<<dim3((unsigned)gx, (unsigned)gy), ST_THREADS, smem, s>>>(tin, a, W, zlo, zhi);
+  kern<<<dim3((unsigned)gx, (unsigned)gy), ST_THREADS, smem, s>>>(tin, a, W, zmask);
   return check_launch();
 }
 
@@ -433,30 +431,21 @@ static int stencil_rows_launch(const StencilArgs &a, const StencilW<T> &W, uint3
              : stencil_rows_on<T, RY, RX, PAT, false>(a, W, zmask, s);
 }
 
-// Zero-weight mask of the taps (bit k set: weight k is zero).
-template <class T>
-void zero_mask(const StencilW<T> &W, int n, uint32_t &lo, uint32_t &hi) {
-  lo = hi = 0;
-  for (int k = 0; k < n; ++k)
-    if (W.w[k] == T(0)) {
-      if (k < 32) lo |= 1u << k; else hi |= 1u << (k - 32);
-    }
-}
-
 template <class T, int RY, int RX>
-int stencil_fast_pat(StencilArgs a, const StencilW<T> &W, cudaStream_t s) {
+int stencil_pat(StencilArgs a, const StencilW<T> &W, cudaStream_t s) {
   constexpr int NT = (2 * RY + 1) * (2 * RX + 1);
   static_assert(NT <= 32, "one mask word");
-  uint32_t lo, hi;
-  zero_mask(W, NT, lo, hi);
+  uint32_t zeros = 0;  // bit k: the weight of tap k is zero
+  for (int k = 0; k < NT; ++k)
+    if (W.w[k] == T(0)) zeros |= 1u << k;
   auto pattern = [&](auto pat) {
     constexpr int PAT = decltype(pat)::value;
-    return a.accumulate ? stencil_fast_launch<T, RY, RX, PAT>(a, W, lo, 0, s)
-                        : stencil_rows_launch<T, RY, RX, PAT>(a, W, lo, s);
+    return a.accumulate ? stencil_onto_launch<T, RY, RX, PAT>(a, W, zeros, s)
+                        : stencil_rows_launch<T, RY, RX, PAT>(a, W, zeros, s);
   };
-  if (lo == 0) return pattern(IC<0>{});
+  if (zeros == 0) return pattern(IC<0>{});
   if constexpr (RY == 1 && RX == 1) {
-    if (lo == ((1u << 0) | (1u << 2) | (1u << 6) | (1u << 8))) return pattern(IC<1>{});
+    if (zeros == ((1u << 0) | (1u << 2) | (1u << 6) | (1u << 8))) return pattern(IC<1>{});
   }
   return pattern(IC<2>{});
 }
@@ -486,10 +475,10 @@ int stencil_typed(StencilArgs a, const void *weights, cudaStream_t s) {
   const int nw = (2 * a.ry + 1) * (2 * a.rx + 1);
   memset(&W, 0, sizeof(W));
   memcpy(W.w, weights, (size_t)nw * sizeof(T));
-  if (a.ry == 1 && a.rx == 1) return stencil_fast_pat<T, 1, 1>(a, W, s);
-  if (a.ry == 0 && a.rx == 1) return stencil_fast_pat<T, 0, 1>(a, W, s);
-  if (a.ry == 1 && a.rx == 0) return stencil_fast_pat<T, 1, 0>(a, W, s);
-  if (a.ry == 2 && a.rx == 2) return stencil_fast_pat<T, 2, 2>(a, W, s);
+  if (a.ry == 1 && a.rx == 1) return stencil_pat<T, 1, 1>(a, W, s);
+  if (a.ry == 0 && a.rx == 1) return stencil_pat<T, 0, 1>(a, W, s);
+  if (a.ry == 1 && a.rx == 0) return stencil_pat<T, 1, 0>(a, W, s);
+  if (a.ry == 2 && a.rx == 2) return stencil_pat<T, 2, 2>(a, W, s);
   const int r = a.ry > a.rx ? a.ry : a.rx;
   if (r <= 1) return stencil_launch<T, 1>(a, W, s);
   if (r <= 2) return stencil_launch<T, 2>(a, W, s);

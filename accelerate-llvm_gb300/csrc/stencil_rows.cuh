@@ -1,6 +1,6 @@
 // stencil_rows.cuh -- how a warp reads a strip of 32 x E columns of one array
-// row into registers, with the boundary columns beside it; shared by the
-// row-streaming stencils of rank 2 (stencil.cu) and rank 3 (stencil3d.cu).
+// row into registers, with the boundary columns beside it, for the row-streaming
+// stencils of stencil.cu.
 #pragma once
 
 #include "stencil_common.cuh"
