@@ -8,8 +8,8 @@
 //     private counters in shared memory, 32 bits per bin while they fit, else
 //     16 bits; the constant multiplies the counts once, at the end;
 //   * permute_private -- every other update of a target that fits in shared
-//     memory: a private copy of the target per CTA, folded into global memory
-//     at the end;
+//     memory, where there are enough of them: a private copy of the target per
+//     CTA, folded into global memory at the end;
 //   * permute_cluster -- for 32-bit integer targets beyond that, up to 8 x 48K
 //     bins: the target is privatised in the DISTRIBUTED shared memory of a
 //     thread-block cluster (each CTA of the cluster holds 1/CL of the bins);
@@ -407,8 +407,8 @@ __global__ void __launch_bounds__(PERM_THREADS, 1) permute_count16(PermArgs a) {
 // target.  L2 takes about 0.15 updates/ns whatever the target and one update
 // per 1.5 ns on a single address; shared memory takes five times that.
 // 2 * 10^7 Float32 values by 5 * 10^4 uniform keys: 0.166 -> 0.050 ms; 6.4 *
-// 10^6 Int64 values by 25,000: 0.057 -> 0.029 ms.  With four updates per bin
-// (the least that comes here) both ways take the time of a call.
+// 10^6 Int64 values by 25,000: 0.057 -> 0.029 ms.  Few updates do not pay for the
+// filling and the folding: see perm_private_pays.
 //
 // 64-bit integer bins are kept as two 32-bit words (all low words first), each
 // updated by a native 32-bit atomic: + adds the low halves, sees its carry in
