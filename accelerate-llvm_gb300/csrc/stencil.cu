@@ -538,6 +538,8 @@ extern "C" int acc_stencil2d_pair(int type, int ry, int rx, const void *wa_w, co
   const int64_t h = ha < hb ? ha : hb, w = wa < wb ? wa : wb;
   if (h == 0 || w == 0) return ACC_OK;
   if (!wa_w || !wb_w || !a_in || !b_in || !out) return ACC_ERR_INVALID;
+  // The second pass's grid, refused before the first pass writes.
+  if (cdiv_h(h, SF_TH) > 65535 || cdiv_h(w, SF_TW) > (1ll << 31) - 1) return ACC_ERR_TOO_LARGE;
   const size_t esz = (type == ACC_F64 || type == ACC_I64) ? 8 : 4;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   Workspace *ws = workspace(s, &st);
