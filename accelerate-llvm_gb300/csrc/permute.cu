@@ -835,7 +835,7 @@ int permute_typed(Workspace *w, PermArgs a, cudaStream_t s) {
   }
   // Four updates per thread from where one each nearly fills the machine; below, more
   // threads are worth more than wider loads (2^17 Float32 max into 2^15 bins: 15.2 us by
-  // four, 7.0 by one; 2^19 into 2^15 15.7 and 21; 2^13 Int64 sums 4.2 and 3.5).
+  // four, 7.0 by one; 2^19 into 2^15 15.7 and 21; 2^12 Int64 sums 4.2 and 3.5).
   if (a.n < (1 << 19)) a.vec = 0;
   int64_t blocks = cdiv_h(a.vec ? cdiv_h(a.n, 4) : a.n, 256);
   if (blocks > (int64_t)d.sms * 16) blocks = (int64_t)d.sms * 16;
