@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(256) foldseg_main(SegArgs a) {
 //     (usually the previous one).
 // An extra tile past the last value closes the segments that end at the very
 // end of the row.  Three launches: the index pre-pass, the tiles and the
-// completion; one for short calls.  Offsets that decrease or leave [0, n] raise
+// completion (two where the last tile takes that over); one for short calls.  Offsets that decrease or leave [0, n] raise
 // ACC_ERR_INDEX; of a tile that holds such offsets only the z of empty segments may
 // have been written, inside of the output.
 // Bound: issue (about 30 thread instructions per value, compensated).  A tile
@@ -298,7 +298,8 @@ struct SegTileArgs {
   struct SegSlot *slots;  // per tile
   const uint64_t *tidx;  // per tile: epoch tag << 35 | first offset index >= the tile start; small: unused
   int small;             // 1: the CTA keeps all the offsets in shared memory; 2: and scans them from the lengths
-  uint32_t *done;  // small: tiles finished (zero between calls)
+  int finish;      // the last tile to get there completes the segments that cross tiles
+  uint32_t *done;  // finish: tiles finished (zero between calls)
   uint32_t *err;
   uint32_t epoch;
 };
@@ -652,7 +653,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a, cons
     if (lane == 0) raise_error(a.err, DEV_ERR_TIMEOUT);
     landed = mbar_wait_sleep(&bar, 0);
   }
-  // The tile's slot; short calls: the last tile to get here completes the
+  // The tile's slot; a.finish: the last tile to get here completes the
   // segments that cross tiles, for all of them.
   auto finish = [&](uint64_t carry, uint64_t first, int64_t first_id, bool boundary) {
     if (tid == 0) {
@@ -662,7 +663,7 @@ foldseg_tile_kernel(const __grid_constant__ CUtensorMap tin, SegTileArgs a, cons
       reinterpret_cast<uint4 *>(a.slots + tile)[0] = q[0];
       reinterpret_cast<uint4 *>(a.slots + tile)[1] = q[1];
     }
-    if (!a.small) return;
+    if (!a.finish) return;
     if (tid == 0) {
       __threadfence();
       s_bad = atomicAdd(a.done, 1u) == (uint32_t)(a.ntiles - 1) ? 2 : 0;
@@ -947,7 +948,7 @@ int launch_foldseg_tile(const CUtensorMap &tin, const SegTileArgs &a, int64_t nt
   smem_attrs_once(kern, (int)(tile + all), attr_done);
   kern<<<(unsigned)ntiles, FT_THREADS, smem, s>>>(tin, a, tin2);
   const int st = check_launch();
-  if (st || a.small) return st;
+  if (st || a.finish) return st;
   foldseg_fix<OP, T, PREC><<<(unsigned)cdiv_h(ntiles, 256), 256, 0, s>>>(a);
   return check_launch();
 }
@@ -1006,6 +1007,10 @@ int foldseg_tile_typed(Workspace *w, const T *in, const void *off, int off64, bo
   a.slots = static_cast<SegSlot *>(w->scratch);
   a.tidx = tidx;
   a.small = small ? (lengths ? 2 : 1) : 0;
+  // Up to as many tiles as a CTA's warps complete at once the last one spares the
+  // completion's launch: 10^6 Float32 values in 62,500 segments 20.5 -> 18.4 us of device
+  // time, 300,000 Int64 in 7,500 18.4 -> 16.4.
+  a.finish = small || ntiles <= FT_THREADS;
   a.done = w->words + W_DONE;
   a.err = w->words + W_ERR;
   a.epoch = ws_next_epoch(w, s);
