@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(256) permute_global(PermArgs a) {
     atomic_combine<OP, T>(out + j, x);
   };
   int64_t e0 = 0;
-  if (a.vec) {
+  if (OP != ACC_MUL && a.vec) {
     // 16-byte loads of four indices and four values.
     for (int64_t v = tid; v < a.n / 4; v += nth) {
       int64_t j[4];
@@ -834,9 +834,13 @@ int permute_typed(Workspace *w, PermArgs a, cudaStream_t s) {
     }
   }
   // Four updates per thread from where one each nearly fills the machine; below, more
-  // threads are worth more than wider loads (2^17 Float32 max into 2^15 bins: 15.2 us by
-  // four, 7.0 by one; 2^19 into 2^15 15.7 and 21; 2^12 Int64 sums 4.2 and 3.5).
-  if (a.n < (1 << 19)) a.vec = 0;
+  // threads are worth more than wider loads.  Compare-and-swap minima and maxima from
+  // 2^19 (2^17 Float32 max into 2^15 bins: 15.2 us by four, 7.0 by one; 2^19 into 2^15 15.7 and
+  // 21), native atomics from 2^21 (2^20 Int64 sums into 200,000 bins 18.2 and 16.5, 2^22 32.6
+  // and 32.8), products, whose retries four at a time add to, never (2^22 Int32 products into
+  // 200,000 bins, uniform keys 108 and 96, 2^24 under Zipf keys 5690 and 5050).
+  constexpr bool loops = is_fp<T>() && (OP == ACC_MIN || OP == ACC_MAX);
+  if (OP == ACC_MUL || a.n < (loops ? 1 << 19 : 1 << 21)) a.vec = 0;
   int64_t blocks = cdiv_h(a.vec ? cdiv_h(a.n, 4) : a.n, 256);
   if (blocks > (int64_t)d.sms * 16) blocks = (int64_t)d.sms * 16;
   permute_global<OP, T><<<(unsigned)blocks, 256, 0, s>>>(a);
