@@ -293,8 +293,10 @@ template <int RY, bool VEC> constexpr int sr_ahead() { return RY == 0 ? 4 : RY =
 template <class T, int RY, bool VEC> constexpr int sr_ctas() {  // 8-byte types: registers without spills
   return sizeof(T) == 8 ? (RY == 2 ? 5 : 8) : RY == 2 ? 8 : VEC ? 14 : 10;
 }
-// 8-byte types are bound by their multiply-adds, of which the rows that two warps share cost some twice
+// 8-byte types are bound by their multiply-adds, of which the rows that two warps share cost some
+// twice; Int64 less so (3x3, 4096 x 4096: 16 rows 72 us, 24 72, 32 74, 48 77)
 template <class T, int RY, bool VEC> constexpr int sr_rows() {
+  if (std::is_same<T, int64_t>::value && RY > 0) return 24;
   return sizeof(T) == 8 ? (RY == 2 ? 96 : 32) : RY == 2 ? 20 : VEC ? 10 : 12;
 }
 
@@ -427,8 +429,13 @@ static int stencil_rows_launch(const StencilArgs &a, const StencilW<T> &W, uint3
   constexpr int E = 16 / (int)sizeof(T);
   const bool vec = aligned16(a.in) && aligned16(a.out) && a.w % E == 0 && a.in_w % E == 0 && a.in_pitch % E == 0 &&
                    a.out_pitch % E == 0;
-  return vec ? stencil_rows_on<T, RY, RX, PAT, true>(a, W, zmask, s)
-             : stencil_rows_on<T, RY, RX, PAT, false>(a, W, zmask, s);
+  // Int64 3x3 and 5x5 take single loads all the same: 4096 x 4096 107 -> 73 us and 206 -> 163,
+  // 8192 x 8192 370 -> 233 and 657 -> 573, from 2048 x 2048 down alike (more rows ahead in 16-byte
+  // loads, 9 to 15, 97 to 117 us; 10 CTAs per SM 87).
+  if constexpr (!(std::is_same<T, int64_t>::value && RY > 0 && RX > 0)) {
+    if (vec) return stencil_rows_on<T, RY, RX, PAT, true>(a, W, zmask, s);
+  }
+  return stencil_rows_on<T, RY, RX, PAT, false>(a, W, zmask, s);
 }
 
 template <class T, int RY, int RX>
